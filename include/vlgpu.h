@@ -165,7 +165,7 @@ int vl_knn_tile(const uint16_t* rows_bf16, int64_t n, int dim_pad, const float* 
 
 /* closest_vectors (ann.py:37-93) as one kernel: the whole budgeted beam search of every query
  * row, with the search queue, the visit queue and the visited set of a row held on chip by
- * one warp.  Replaces, per iteration, pop_n_ids + search_from_seeds + two Queue.insert +
+ * one CTA.  Replaces, per iteration, pop_n_ids + search_from_seeds + two Queue.insert +
  * add_new_to_seen_.  The caller (the Python driver) checks the two flag arrays afterwards to
  * learn whether the reference's batch-wide loop would have stopped earlier. */
 typedef struct vl_beam_params {
@@ -203,11 +203,10 @@ typedef struct vl_beam_params {
     uint32_t* group_full;      /* [groups]: set when some row of the batch never popped a MAXINT */
     int32_t* status;
     unsigned long long* memo;  /* [memo_slots, memo_entries] scratch, any contents (see vl_beam_search_plan) */
-    int64_t memo_slots;        /* rows in flight the scratch was sized for: >= blocks * warps_per_block of the plan */
+    int64_t memo_slots;        /* rows in flight the scratch was sized for: >= blocks * rows_per_block of the plan */
     unsigned long long* stats; /* optional [16] counters (added to): [1] gathered candidates, [2] search-queue merges,
-                                  [3] visit-queue merges, [4] class-A candidates, [5] class-B rounds, [6] rows, [7] iterations, [8..13] warp cycles spent in: pop +
-                                  neighbour ids, memo probe, gather, memo update, search-queue merge, visit-queue merge */
-    int32_t flags;             /* bit 0: also accumulate the per-phase cycle counters of `stats` */
+                                  [3] visit-queue merges, [4] class-A candidates, [5] class-B rounds, [6] rows, [7] iterations */
+    int32_t flags;             /* ignored (a row's phases overlap, so they have no cycle counters of their own) */
     int32_t reserved;
     unsigned long long* row_ticket; /* optional device counter, zero at launch: warps then draw their next row from it
                                   (rows that take unequal time no longer wait for a fixed partner); NULL = fixed stride */
@@ -218,16 +217,16 @@ typedef struct vl_beam_params {
 
 int vl_beam_search(const vl_beam_params* params, void* stream);
 
-/* Bytes of shared memory one warp (= one query row in flight) of vl_beam_search needs for the
- * given shape, the warps per CTA and the CTAs it will launch.  blocks * warps_per_block is the
- * number of rows in flight, i.e. the memo_slots a distance memo must provide.
+/* Bytes of shared memory one query row in flight of vl_beam_search needs for the given shape, the rows
+ * per CTA and the CTAs it will launch.  blocks * rows_per_block is the number of rows in flight, i.e.
+ * the memo_slots a distance memo must provide.
  *
  * The memo: during one row's search the same candidate id comes back many times (neighbour
  * lists of nearby nodes overlap; the reference recomputes its distance every time).  With a
  * memo the kernel keeps id -> distance of the row's recent candidates in a 2-way table in
  * global memory (L2-resident) and gathers only the ids it has not met: same bits, a fraction
  * of the gathers. */
-int vl_beam_search_plan(const vl_beam_params* params, int* smem_per_warp, int* warps_per_block, int* blocks);
+int vl_beam_search_plan(const vl_beam_params* params, int* smem_per_row, int* rows_per_block, int* blocks);
 
 #ifdef __cplusplus
 }

@@ -1,0 +1,50 @@
+// Fused beam search with two warps per query row, 16 rows in flight per SM: launches of many rows.
+//
+// A row's iteration is a chain of memory round trips and queue steps, so a launch is bound by latency
+// at the number of rows that can be in flight.  That number is bound in turn by the rows' memos
+// (64 KB each at a build's 30,720 evaluations, 155 MB in all, already more than the 126 MB L2), not by
+// registers: a second warp per row halves the id, memo and gather phases and runs the two queue steps side
+// by side at 64 registers per thread, without another row's memo.  Build rounds, ms, one warp per row with
+// the queue merges of before (128 registers) / this, on one B200:
+//   1,000,000 x 128, lists of 96 from near neighbours: 660 / 526
+//   60,007 x 768, lists of 192:                        155 / 121
+//   150,000 x 128, rounds 2 and 3:                  98, 97 / 76, 78
+// 10,000 searches of 1,000,000 x 128: 6.6 / 5.3; 2,500 of 200,000 x 256: 2.33 / 1.55.  12 rows per SM at 80
+// registers (two gather steps in flight): 541, 119, 81; one warp per row with the same queue step at 16 rows per
+// SM: 528, 137, 75, at 24 rows per SM: 740, 144, 108.
+#include "vl_beam_team.cuh"
+
+namespace {
+
+template <int LPR, int JP, int JU, int METRIC, bool ALIGNED>
+int pair_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)
+{
+    auto kernel = beam_team_kernel<LPR, JP, JU, METRIC, ALIGNED, 2>;
+    const TeamSmem lay = team_layout(p.pvc * p.graph_w, p.sq_len, p.vq_len, p.seen_cap, LPR * JP * 16, p.memo ? p.memo_entries : 0, false);
+    int dev = 0, max_smem = 0, per_sm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    VL_CHECK_ARG(e == cudaSuccess, "vl_beam_search: %s", cudaGetErrorString(e));
+    VL_CHECK_ARG(lay.total <= max_smem, "vl_beam_search: one row needs %d bytes of shared memory, the device offers %d", lay.total, max_smem);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lay.total);
+    VL_CHECK_ARG(e == cudaSuccess, "vl_beam_search: %s", cudaGetErrorString(e));
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 64, lay.total);
+    VL_CHECK_ARG(e == cudaSuccess && per_sm > 0, "vl_beam_search: occupancy query failed");
+    const int64_t resident = (int64_t)vl_sm_count() * per_sm;   // one resident wave; further rows are drawn as CTAs finish
+    const int grid = (int)(p.rows < resident ? p.rows : resident);
+    *blocks = grid;
+    *smem = lay.total;
+    if (!launch) return 0;
+    VL_CHECK_ARG(!p.memo || p.memo_slots >= grid, "vl_beam_search: memo has %lld slots, the launch keeps %d rows in flight",
+                 (long long)p.memo_slots, grid);
+    kernel<<<grid, 64, lay.total, stream>>>(p, lay, row_order, nullptr);
+    VL_CHECK_LAUNCH("beam_team_kernel");
+    return 0;
+}
+
+}  // namespace
+
+int vl_beam_pair_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)
+{
+    VL_BEAM_DISPATCH(p, pair_launch, p, row_order, launch, blocks, smem, stream);
+}

@@ -30,10 +30,9 @@ FUSED_MAX_SMEM_PER_ROW = 200 * 1024
 # launching stream) and its count of distance evaluations: the benchmark's roofline figures.
 PROFILE = None
 PROFILE_TAG = "search"     # which phase the launches being profiled belong to (generate_ann sets it per round)
-# When set to an int64 CUDA tensor of 16 zeros, the fused kernel adds its work counters and
-# per-phase warp cycles to it (layout: `stats` in include/vlgpu.h).
+# When set to an int64 CUDA tensor of 16 zeros, the fused kernel adds its work counters to it
+# (layout: `stats` in include/vlgpu.h).
 STATS = None
-STATS_TIMERS = False
 
 
 def _metric_of(config: Dict):
@@ -47,7 +46,7 @@ def _fused_shape_ok(vectors: Tensor, beam_w: int, sq_len: int, sq_cap: int, conf
     vq_len = config["visit_queue_factor"] * config["beam_size"]
     m = pvc * beam_w
     e = config["exclude_factor"] * vq_len
-    smem = 10 * m + 16 * sq_len + 16 * vq_len + 4 * 6 * max(e, 16) + 4 * vectors.size(1) + 512
+    smem = 14 * m + 16 * sq_len + 16 * vq_len + 4 * 6 * max(e, 16) + 4 * 1024 + 512
     return (vectors.size(1) % 4 == 0 and vectors.data_ptr() % 16 == 0 and 1 <= pvc <= 32 and pvc <= vq_len
             and sq_cap == sq_len + m and sq_len <= 4096 and smem <= FUSED_MAX_SMEM_PER_ROW
             and config["speculative_readahead"] >= 1)
@@ -114,21 +113,21 @@ def _launch_beam(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_len
     p.memo_entries = 0
     p.memo_slots = 0
     p.stats = stats.data_ptr() if stats is not None else 0
-    p.flags = 1 if (stats is not None and stats is STATS and STATS_TIMERS) else 0
-    # rows differ in the work they take: warps draw their next row from a counter instead of a fixed stride
+    p.flags = 0
+    # rows differ in the work they take: CTAs draw their next row from a counter instead of a fixed stride
     ticket = torch.zeros(1, dtype=torch.int64, device=vectors.device) if config.get("row_ticket", True) else None
     p.row_ticket = ticket.data_ptr() if ticket is not None else 0
     if config.get("memo", True):
         # id -> distance memo of each row in flight (scratch; the kernel clears a row's slice)
-        smem, warps, blocks = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
-        check(lib().vl_beam_search_plan(ctypes.byref(p), ctypes.byref(smem), ctypes.byref(warps), ctypes.byref(blocks)),
+        smem, per_block, blocks = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
+        check(lib().vl_beam_search_plan(ctypes.byref(p), ctypes.byref(smem), ctypes.byref(per_block), ctypes.byref(blocks)),
               "vl_beam_search_plan")
         entries = int(config.get("memo_entries", 0))
         if entries <= 0:
             entries = 1024        # measured on 1M x 128: 8192 entries per row at E=320 (24*E) is the knee
             while entries < 24 * p.seen_cap and entries < 16384:
                 entries *= 2
-        slots = max(1, warps.value * blocks.value)
+        slots = max(1, per_block.value * blocks.value)
         memo = _memo_buffer(vectors.device, slots * entries)
         p.memo = memo.data_ptr()
         p.memo_entries = entries
