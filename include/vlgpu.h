@@ -217,9 +217,20 @@ typedef struct vl_beam_params {
 
 int vl_beam_search(const vl_beam_params* params, void* stream);
 
+/* vl_beam_search with one more, optional, argument.
+ *
+ * arrivals [n_checks + 1], zeroed: the launch may end where the reference's loop leaves (ann.py:85-91), at
+ * the first check at which no row of the batch changed.  It does so only if the rows are one batch and
+ * all in flight at once, out_cols >= sq_len + pvc * graph_w and dump_last == 0; it then stores that
+ * iteration in arrivals[n_checks] and every row holds head + that iteration's candidates as with
+ * dump_last.  Otherwise arrivals[n_checks] stays 0 and the launch is vl_beam_search's.  A wait between
+ * rows that runs out (2 s) sets VL_STATUS_TIMEOUT in *status. */
+int vl_beam_search_rows(const vl_beam_params* params, uint32_t* arrivals, void* stream);
+
 /* Bytes of shared memory one query row in flight of vl_beam_search needs for the given shape, the rows
  * per CTA and the CTAs it will launch.  blocks * rows_per_block is the number of rows in flight, i.e.
- * the memo_slots a distance memo must provide.
+ * the memo_slots a distance memo must provide; 0 blocks: the rows keep their memo on chip and the launch
+ * needs no scratch.
  *
  * The memo: during one row's search the same candidate id comes back many times (neighbour
  * lists of nearby nodes overlap; the reference recomputes its distance every time).  With a

@@ -1,0 +1,65 @@
+"""The launches of the fused beam search - a CTA of several warps per row when rows are few, two warps per
+row beyond - against the step-by-step operator path, at the row counts where the launch changes."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def rows_of(seed, count, dim, metric):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(seed)
+    x = torch.randn((count, dim), generator=g, device=DEV)
+    return torch.nn.functional.normalize(x, dim=1) if metric == "cosine" else (x * 40).round_()
+
+
+def search_both_ways(ann, queries):
+    """The whole queues (ids, distances, columns behind the head too) and the loop counts: fused, operator path."""
+    from vectorlink_gpu.ann import closest_vectors
+    out = []
+    for stepwise in (False, True):
+        ann.configuration["stepwise"] = stepwise
+        queue = ann.search(queries)
+        out.append((queue.indices.clone(), queue.distances.clone(), closest_vectors.last_count))
+    ann.configuration["stepwise"] = False
+    return out
+
+
+# one row per SM (16 or 8 warps), two (8), four (4), eight (2), more (two warps, memo in global memory); 148 SMs
+@pytest.mark.parametrize("count", [1, 2, 5, 148, 149, 296, 297, 592, 593, 1184, 1185, 2500])
+@pytest.mark.parametrize("metric,dim,degree", [("cosine", 64, 16), ("l2", 100, 24), ("cosine", 768, 64)])
+def test_every_split_of_a_row_gives_the_operator_path_queues(count, metric, dim, degree, built_lib):
+    from vectorlink_gpu import ANN, _lib
+    if degree == 64 and count > 300:
+        pytest.skip("the operator path takes long at this width")
+    ann = ANN(vectors=rows_of(1, 3001, dim, metric), beam_size=degree, visit_queue_factor=2, recall_search_queue_factor=2,
+              metric=metric, init="knn_tile", optimization_loops=1)
+    (fused, steps) = search_both_ways(ann, rows_of(2, count, dim, metric))
+    assert torch.equal(fused[0], steps[0]) and torch.equal(fused[1], steps[1])
+    assert fused[2] == steps[2]
+    assert _lib.read_status(DEV) == 0
+
+
+def test_a_batch_that_stops_early_ends_together(built_lib):
+    """Few rows stop at the reference's check: one launch, no second run up to it."""
+    import vectorlink_gpu.ann as A
+    ann = A.ANN(vectors=rows_of(3, 4000, 64, "cosine"), beam_size=16, visit_queue_factor=2, recall_search_queue_factor=2,
+                init="knn_tile", optimization_loops=1)
+    k_none = A.loop_bounds(ann.configuration)[0]
+    early = 0
+    for count in (1, 2, 3):
+        for seed in range(4):
+            queries = rows_of(10 + seed, count, 64, "cosine")
+            A.PROFILE = []
+            try:
+                ann.search(queries)
+                launches = len(A.PROFILE)
+            finally:
+                A.PROFILE = None
+            (fused, steps) = search_both_ways(ann, queries)
+            assert torch.equal(fused[0], steps[0]) and torch.equal(fused[1], steps[1]) and fused[2] == steps[2]
+            assert launches == 1
+            early += steps[2] <= k_none
+    assert early > 0

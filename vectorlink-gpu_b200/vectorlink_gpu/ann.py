@@ -68,7 +68,8 @@ def loop_bounds(config: Dict) -> Tuple[int, int, int]:
 
 
 def _launch_beam(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_len, out_ids, out_dist, out_cols,
-                 config, n_iters, dump_last, exclude, self_base, group_rows, flags, full, stats=None, group_row0=0):
+                 config, n_iters, dump_last, exclude, self_base, group_rows, flags, full, stats=None, group_row0=0,
+                 arrivals=None):
     pvc = config["parallel_visit_count"]
     if stats is None:
         stats = STATS
@@ -136,7 +137,7 @@ def _launch_beam(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_len
         start = torch.cuda.Event(enable_timing=True)
         end = torch.cuda.Event(enable_timing=True)
         start.record()
-    check(lib().vl_beam_search(ctypes.byref(p), stream_of(vectors)), "vl_beam_search")
+    check(lib().vl_beam_search_rows(ctypes.byref(p), ptr(arrivals), stream_of(vectors)), "vl_beam_search_rows")
     if PROFILE is not None:
         end.record()
         k_none = (p.seen_cap + pvc - 1) // pvc + 1
@@ -190,9 +191,14 @@ def _fused_batches(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_l
     nc = max(n_checks, 1)
     ng = max(total_groups, 1)
     # one buffer for both flag arrays: one all-reduce, one read-back
-    flag_buf = torch.zeros(ng * nc + ng, dtype=torch.int32, device=dev)
+    flag_buf = torch.zeros(ng * nc + ng + nc + 1, dtype=torch.int32, device=dev)
     flags = flag_buf[: ng * nc].view(ng, nc)
-    full = flag_buf[ng * nc:]
+    full = flag_buf[ng * nc: ng * nc + ng]
+    # one batch whose rows are all in flight at once may end together at the check at which the reference
+    # leaves (the kernel then stores that iteration in the last word) instead of being run again up to it
+    together = {}
+    if rows and reduce_group is None and ng == 1 and out_cols == sq_cap and out_ids.is_cuda and out_ids.is_contiguous():
+        together = {"arrivals": flag_buf[ng * nc + ng:]}
     if rows == 0 and reduce_group is None:
         return []
     # a caller that wants to know how useful the distance memo is on this graph (generate_ann's
@@ -202,7 +208,8 @@ def _fused_batches(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_l
         counters = torch.zeros(24, dtype=torch.int64, device=dev)
     if rows:
         _launch_beam(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_len, out_ids, out_dist, out_cols,
-                     config, n_max, False, exclude, self_base, group_rows, flags, full, counters, group_row0)
+                     config, n_max, False, exclude, self_base, group_rows, flags, full, counters, group_row0,
+                     **together)
     if reduce_group is not None:
         import torch.distributed as dist
         with nvtx_range("vl.flags_allreduce"):
@@ -211,7 +218,8 @@ def _fused_batches(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_l
         return []
     host = flag_buf.cpu()
     flags_h = host[: ng * nc].view(ng, nc).tolist()
-    full_h = host[ng * nc:].tolist()
+    full_h = host[ng * nc: ng * nc + ng].tolist()
+    ended = int(host[-1])
     if counters is not None:
         if STATS is not None:
             shared = min(STATS.numel(), counters.numel())
@@ -228,6 +236,10 @@ def _fused_batches(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_l
             continue
         counts.append(end)
         if end > k_none:
+            continue
+        if ended:
+            # the rows hold their heads and that iteration's candidates
+            sort_pairs_(out_ids, out_dist, dedup=True)
             continue
         # the reference left at check iteration `end`: redo the batch up to it; the last insert
         # is a whole-row sort so that the columns behind `length` match too
