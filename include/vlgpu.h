@@ -171,7 +171,7 @@ int vl_knn_tile(const uint16_t* rows_bf16, int64_t n, int dim_pad, const float* 
 typedef struct vl_beam_params {
     const float* vectors;      /* [n, dim] */
     int64_t n;
-    int32_t dim;               /* multiple of 4, rows 16-byte aligned */
+    int32_t dim;               /* any; multiples of 4 with 16-byte aligned rows take 128-bit loads */
     int32_t metric;
     const int32_t* graph;      /* [n, graph_w]  (`beams` of the reference) */
     int32_t graph_w;

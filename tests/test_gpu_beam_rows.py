@@ -63,3 +63,30 @@ def test_a_batch_that_stops_early_ends_together(built_lib):
             assert launches == 1
             early += steps[2] <= k_none
     assert early > 0
+
+
+@pytest.mark.parametrize("metric", ["cosine", "l2"])
+@pytest.mark.parametrize("dim,offset", [(1, 0), (3, 0), (50, 0), (127, 0), (255, 0), (511, 0), (1023, 0), (1027, 0), (64, 1), (96, 3)])
+def test_rows_without_whole_aligned_chunks_give_the_operator_path_results(dim, offset, metric, built_lib):
+    """Dimensions that are no multiple of four, and rows whose storage starts off a 16-byte boundary: searches of few
+    and of many rows, a build, and the same build without the padded copy."""
+    import vectorlink_gpu.ann as A
+    n = 1500
+    store = torch.empty(n * dim + offset, device=DEV)
+    vectors = store[offset:].view(n, dim)
+    vectors.copy_(rows_of(5, n, dim, metric))
+    assert vectors.is_contiguous() and (dim % 4 or vectors.data_ptr() % 16)
+    config = dict(beam_size=8, visit_queue_factor=2, recall_search_queue_factor=2, metric=metric, optimization_loops=1)
+    ann = A.ANN(vectors=vectors, **config)
+    plain = A.generate_ann(vectors, dict(ann.configuration, stepwise=True))
+    assert torch.equal(ann.beams, plain[0]) and torch.equal(ann.distances, plain[1])
+    keep = A._chunked_rows
+    A._chunked_rows = lambda v: v
+    try:
+        uncopied = A.generate_ann(vectors, ann.configuration)
+    finally:
+        A._chunked_rows = keep
+    assert torch.equal(uncopied[0], plain[0]) and torch.equal(uncopied[1], plain[1])
+    for count in (3, 1300):
+        (fused, steps) = search_both_ways(ann, rows_of(6, count, dim, metric))
+        assert torch.equal(fused[0], steps[0]) and torch.equal(fused[1], steps[1]) and fused[2] == steps[2]

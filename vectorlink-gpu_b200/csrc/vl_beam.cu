@@ -38,8 +38,6 @@ int beam_dispatch(const vl_beam_params* pp, unsigned int* arrivals, int* blocks,
     VL_CHECK_ARG(p.vectors && p.graph && p.queries && p.seed_ids && p.seed_dist && p.out_ids && p.out_dist &&
                  p.changed_flags && p.group_full && p.status, "vl_beam_search: null pointer");
     VL_CHECK_ARG(p.n > 0 && p.rows >= 0 && p.dim > 0, "vl_beam_search: bad size");
-    VL_CHECK_ARG(p.dim % 4 == 0 && ((uintptr_t)p.vectors | (uintptr_t)p.queries) % 16 == 0,
-                 "vl_beam_search: needs dim %% 4 == 0 and 16-byte aligned rows (dim=%d)", p.dim);
     VL_CHECK_ARG(p.metric == VL_METRIC_COSINE || p.metric == VL_METRIC_SQL2, "vl_beam_search: unknown metric %d", p.metric);
     VL_CHECK_ARG(p.pvc >= 1 && p.pvc <= 32, "vl_beam_search: parallel_visit_count %d outside 1..32", p.pvc);
     VL_CHECK_ARG(p.graph_w >= 1 && p.sq_len >= 1 && p.sq_len <= 4096, "vl_beam_search: bad queue shape");

@@ -39,7 +39,7 @@ def _metric_of(config: Dict):
     return config.get("metric", "cosine")
 
 
-def _fused_shape_ok(vectors: Tensor, beam_w: int, sq_len: int, sq_cap: int, config: Dict) -> bool:
+def _fused_queue_ok(beam_w: int, sq_len: int, sq_cap: int, config: Dict) -> bool:
     """The fused kernel models a queue as "the `length` best of head + candidates", which is
     what Queue.insert computes when capacity == length + candidates per iteration."""
     pvc = config["parallel_visit_count"]
@@ -47,9 +47,14 @@ def _fused_shape_ok(vectors: Tensor, beam_w: int, sq_len: int, sq_cap: int, conf
     m = pvc * beam_w
     e = config["exclude_factor"] * vq_len
     smem = 14 * m + 16 * sq_len + 16 * vq_len + 4 * 6 * max(e, 16) + 4 * 1024 + 512
-    return (vectors.size(1) % 4 == 0 and vectors.data_ptr() % 16 == 0 and 1 <= pvc <= 32 and pvc <= vq_len
-            and sq_cap == sq_len + m and sq_len <= 4096 and smem <= FUSED_MAX_SMEM_PER_ROW
-            and config["speculative_readahead"] >= 1)
+    return (1 <= pvc <= 32 and pvc <= vq_len and sq_cap == sq_len + m and sq_len <= 4096 and m <= 65535
+            and smem <= FUSED_MAX_SMEM_PER_ROW and config["speculative_readahead"] >= 1)
+
+
+def _fused_shape_ok(vectors: Tensor, beam_w: int, sq_len: int, sq_cap: int, config: Dict) -> bool:
+    """Queues as above and rows of whole, aligned 16-byte chunks: the kernel's 128-bit row loads."""
+    return (vectors.size(1) % 4 == 0 and vectors.data_ptr() % 16 == 0
+            and _fused_queue_ok(beam_w, sq_len, sq_cap, config))
 
 
 def loop_bounds(config: Dict) -> Tuple[int, int, int]:
@@ -307,7 +312,7 @@ def closest_vectors(query_vecs: Tensor, search_queue: Queue, vectors: Tensor, be
     (batch_size, queue_capacity) = search_queue.size()
     sq_len = search_queue.length
     force_stepwise = bool(config.get("stepwise", False))
-    if force_stepwise or not _fused_shape_ok(vectors, beams.size(1), sq_len, queue_capacity, config) or batch_size == 0:
+    if force_stepwise or not _fused_queue_ok(beams.size(1), sq_len, queue_capacity, config) or batch_size == 0:
         closest_vectors.last_count = closest_vectors_stepwise(query_vecs, search_queue, vectors, beams, config, exclude)
         return True
     if exclude is not None:
@@ -362,6 +367,20 @@ def _gather_row_blocks(buf: Tensor, per: int, group) -> None:
         dist.all_gather([buf[r * per:(r + 1) * per] for r in range(world)], mine.clone(), group=group)
 
 
+def _chunked_rows(vectors: Tensor) -> Tensor:
+    """The rows zero-padded to whole, aligned 16-byte chunks, for a build that gathers each of them thousands
+    of times; the rows themselves where a copy would take more than a quarter of the free memory (the
+    kernels then load them element by element).  Elements at or past the dimension read as zero in every
+    distance, so no result changes."""
+    (n, dim) = vectors.size()
+    pad = (dim + 3) // 4 * 4
+    if n == 0 or 4 * n * pad > torch.cuda.mem_get_info(vectors.device)[0] // 4:
+        return vectors
+    out = torch.zeros((n, pad), dtype=vectors.dtype, device=vectors.device)
+    out[:, :dim] = vectors
+    return out
+
+
 def generate_ann(vectors: Tensor, config: Dict, group=None) -> Tuple[Tensor, Tensor]:
     """ann.py:109-193: circulant start graph of width W = beam_size * beam_queue_factor, then up
     to `optimization_loops` rounds of: beam-search every node from its current neighbours
@@ -389,7 +408,9 @@ def generate_ann(vectors: Tensor, config: Dict, group=None) -> Tuple[Tensor, Ten
     remaining_capacity = queue_length * config["parallel_visit_count"]
     capacity = queue_length + remaining_capacity
     batch_size = config["batch_size"]
-    fused = not config.get("stepwise", False) and _fused_shape_ok(vectors, queue_length, queue_length, capacity, config)
+    fused = not config.get("stepwise", False) and _fused_queue_ok(queue_length, queue_length, capacity, config)
+    if fused and vectors.is_cuda and not _fused_shape_ok(vectors, queue_length, queue_length, capacity, config):
+        vectors = _chunked_rows(vectors)
     world, rank = 1, 0
     if group is not None:
         import torch.distributed as dist
@@ -772,7 +793,7 @@ class ANN:
         beams = self.beams.contiguous()
         entry_sample = int(config.get("search_entry_sample", 0))
         fused_ok = (query.size(0) > 0 and not config.get("stepwise", False)
-                    and _fused_shape_ok(self.vectors, beams.size(1), queue_size, queue_size + extra_capacity, config))
+                    and _fused_queue_ok(beams.size(1), queue_size, queue_size + extra_capacity, config))
         if entry_sample > 0 and query.size(0) > 0:
             # entry points from the tensor-core pass instead of circulant seeds
             seeds = self._entry_seeds(query)
