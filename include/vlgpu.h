@@ -217,7 +217,11 @@ typedef struct vl_beam_params {
 
 int vl_beam_search(const vl_beam_params* params, void* stream);
 
-/* vl_beam_search with one more, optional, argument.
+/* vl_beam_search with two more, optional, arguments.
+ *
+ * row_order [rows]: a permutation of 0..rows-1 on the device in which rows are taken (NULL = by row
+ * number; launches that keep all rows in flight ignore it).  The results are the same row by row; rows
+ * that are close in the index and taken together share the candidate rows they gather.
  *
  * arrivals [n_checks + 1], zeroed: the launch may end where the reference's loop leaves (ann.py:85-91), at
  * the first check at which no row of the batch changed.  It does so only if the rows are one batch and
@@ -225,7 +229,13 @@ int vl_beam_search(const vl_beam_params* params, void* stream);
  * iteration in arrivals[n_checks] and every row holds head + that iteration's candidates as with
  * dump_last.  Otherwise arrivals[n_checks] stays 0 and the launch is vl_beam_search's.  A wait between
  * rows that runs out (2 s) sets VL_STATUS_TIMEOUT in *status. */
-int vl_beam_search_rows(const vl_beam_params* params, uint32_t* arrivals, void* stream);
+int vl_beam_search_rows(const vl_beam_params* params, const int64_t* row_order, uint32_t* arrivals, void* stream);
+
+/* Sort keys for such an order when the rows searched are the indexed vectors [row_lo, row_hi)
+ * themselves: keys_out[x - row_lo] = (smallest hashed id within two steps of x in graph [n, w]) << 32 |
+ * (within one step), MAXINT entries skipped.  near: scratch, n words. */
+int vl_locality_keys(const int32_t* graph, int64_t n, int w, int64_t row_lo, int64_t row_hi, uint32_t* near,
+                     long long* keys_out, void* stream);
 
 /* Bytes of shared memory one query row in flight of vl_beam_search needs for the given shape, the rows
  * per CTA and the CTAs it will launch.  blocks * rows_per_block is the number of rows in flight, i.e.

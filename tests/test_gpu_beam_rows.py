@@ -90,3 +90,39 @@ def test_rows_without_whole_aligned_chunks_give_the_operator_path_results(dim, o
     for count in (3, 1300):
         (fused, steps) = search_both_ways(ann, rows_of(6, count, dim, metric))
         assert torch.equal(fused[0], steps[0]) and torch.equal(fused[1], steps[1]) and fused[2] == steps[2]
+
+
+def test_row_order_of_a_build_changes_nothing(built_lib):
+    import vectorlink_gpu.ann as A
+    vectors = rows_of(7, 5000, 48, "cosine")
+    config = dict(A.ANN(vectors=vectors[:64].contiguous(), beam_size=8).configuration, batch_size=1700)
+    keep = A.ORDER_MIN_ROWS
+    graphs = []
+    try:
+        for least in (keep, 1):
+            A.ORDER_MIN_ROWS = least
+            graphs.append(A.generate_ann(vectors, dict(config, memo=True)))
+    finally:
+        A.ORDER_MIN_ROWS = keep
+    assert torch.equal(graphs[0][0], graphs[1][0]) and torch.equal(graphs[0][1], graphs[1][1])
+
+
+@pytest.mark.parametrize("n,w,lo,hi", [(1, 1, 0, 1), (50, 7, 10, 50), (3000, 96, 0, 3000)])
+def test_locality_keys(n, w, lo, hi, built_lib):
+    from vectorlink_gpu._lib import lib, ptr, stream_of
+    rng = np.random.default_rng(n)
+    graph = rng.integers(0, n, size=(n, w)).astype(np.int32)
+    graph[rng.random((n, w)) < 0.2] = 2147483647
+    g = torch.from_numpy(graph).to(DEV)
+    near = torch.empty(n, dtype=torch.int32, device=DEV)
+    keys = torch.empty(hi - lo, dtype=torch.int64, device=DEV)
+    assert lib().vl_locality_keys(ptr(g), n, w, lo, hi, ptr(near), ptr(keys), stream_of(g)) == 0
+    hashed = (np.arange(n, dtype=np.uint64) * 2654435761 & 0x7fffffff).astype(np.int64)
+
+    def smallest(values):
+        padded = np.append(values, 1 << 40)
+        return np.minimum(values, padded[np.where(graph < n, graph, n)].min(axis=1))
+
+    one = smallest(hashed)
+    two = smallest(one)
+    assert np.array_equal(keys.cpu().numpy(), ((two << 32) | one)[lo:hi])

@@ -31,7 +31,8 @@
 
 namespace {
 
-int beam_dispatch(const vl_beam_params* pp, unsigned int* arrivals, int* blocks, int* smem, bool launch, cudaStream_t stream)
+int beam_dispatch(const vl_beam_params* pp, const int64_t* row_order, unsigned int* arrivals, int* blocks, int* smem, bool launch,
+                  cudaStream_t stream)
 {
     VL_CHECK_ARG(pp, "vl_beam_search: null params");
     const vl_beam_params& p = *pp;
@@ -55,7 +56,7 @@ int beam_dispatch(const vl_beam_params* pp, unsigned int* arrivals, int* blocks,
     *blocks = *smem = 0;
     if (p.rows == 0) return 0;
     if (vl_beam_team_fits(p)) return launch ? vl_beam_team_launch(p, arrivals, stream) : 0;   // no scratch: *blocks stays 0
-    return vl_beam_pair_launch(p, nullptr, launch, blocks, smem, stream);
+    return vl_beam_pair_launch(p, row_order, launch, blocks, smem, stream);
 }
 
 }  // namespace
@@ -63,19 +64,19 @@ int beam_dispatch(const vl_beam_params* pp, unsigned int* arrivals, int* blocks,
 extern "C" int vl_beam_search(const vl_beam_params* params, void* stream)
 {
     int blocks, smem;
-    return beam_dispatch(params, nullptr, &blocks, &smem, true, (cudaStream_t)stream);
+    return beam_dispatch(params, nullptr, nullptr, &blocks, &smem, true, (cudaStream_t)stream);
 }
 
-extern "C" int vl_beam_search_rows(const vl_beam_params* params, uint32_t* arrivals, void* stream)
+extern "C" int vl_beam_search_rows(const vl_beam_params* params, const int64_t* row_order, uint32_t* arrivals, void* stream)
 {
     int blocks, smem;
-    return beam_dispatch(params, arrivals, &blocks, &smem, true, (cudaStream_t)stream);
+    return beam_dispatch(params, row_order, arrivals, &blocks, &smem, true, (cudaStream_t)stream);
 }
 
 extern "C" int vl_beam_search_plan(const vl_beam_params* params, int* smem_per_row, int* rows_per_block, int* blocks)
 {
     int b = 0, s = 0;
-    int rc = beam_dispatch(params, nullptr, &b, &s, false, nullptr);
+    int rc = beam_dispatch(params, nullptr, nullptr, &b, &s, false, nullptr);
     if (rc) return rc;
     if (smem_per_row) *smem_per_row = s;
     if (rows_per_block) *rows_per_block = 1;
