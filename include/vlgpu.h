@@ -163,6 +163,13 @@ int vl_knn_prepare(const float* vectors, int64_t n, int dim, uint16_t* bf16_out,
 int vl_knn_tile(const uint16_t* rows_bf16, int64_t n, int dim_pad, const float* sqnorm, int64_t row_lo, int64_t row_hi,
                 int64_t cand_lo, int64_t cand_hi, int segments, int32_t* out_ids, int* status, void* stream);
 
+/* vl_knn_tile with the same lists, for few rows: every segment is divided over `parts` (1..32) work items so
+ * that more SMs take part, and a second kernel joins their lists.  scratch (parts > 1): 64-bit words
+ * [row_hi - row_lo, segments, parts, VL_KNN_TILE_LISTS, VL_KNN_TILE_K]. */
+int vl_knn_tile_parts(const uint16_t* rows_bf16, int64_t n, int dim_pad, const float* sqnorm, int64_t row_lo,
+                      int64_t row_hi, int64_t cand_lo, int64_t cand_hi, int segments, int parts,
+                      unsigned long long* scratch, int32_t* out_ids, int* status, void* stream);
+
 /* closest_vectors (ann.py:37-93) as one kernel: the whole budgeted beam search of every query
  * row, with the search queue, the visit queue and the visited set of a row held on chip by
  * one CTA.  Replaces, per iteration, pop_n_ids + search_from_seeds + two Queue.insert +

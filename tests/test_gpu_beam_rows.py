@@ -126,3 +126,20 @@ def test_locality_keys(n, w, lo, hi, built_lib):
     one = smallest(hashed)
     two = smallest(one)
     assert np.array_equal(keys.cpu().numpy(), ((two << 32) | one)[lo:hi])
+
+
+@pytest.mark.parametrize("rows,cands,segments,parts", [((0, 1), (0, 3000), 1, 2), ((0, 129), (0, 3000), 1, 32),
+                                                       ((2990, 3000), (100, 2777), 2, 5), ((7, 300), (0, 255), 1, 3)])
+@pytest.mark.parametrize("dim", [64, 200])
+def test_divided_segments_give_the_same_proposals(rows, cands, segments, parts, dim, built_lib):
+    from vectorlink_gpu import knn_tile
+    rows_bf16, norms = knn_tile.prepare(rows_of(8, 3000, dim, "l2"), want_norms=True)
+    keep = knn_tile._parts
+    got = []
+    try:
+        for count in (1, parts):
+            knn_tile._parts = lambda *a: count
+            got.append(knn_tile.proposals(rows_bf16, norms, rows, cands, segments).clone())
+    finally:
+        knn_tile._parts = keep
+    assert torch.equal(got[0], got[1])

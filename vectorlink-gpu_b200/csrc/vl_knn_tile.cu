@@ -189,7 +189,10 @@ struct KnnArgs {
     int64_t cand_lo, cand_hi; // candidates offered to every row
     int segments;             // the candidate range is cut into this many parts, each with its own top-k
     int64_t seg_len;          // candidates per part (a multiple of 256)
-    int32_t* out_ids;         // [row_hi - row_lo, segments, kLists, kTopK]
+    int parts;                // work items a segment is divided into
+    int64_t part_len;         // candidates per work item (a multiple of 256)
+    int32_t* out_ids;         // [row_hi - row_lo, segments, kLists, kTopK]; written when parts == 1
+    vl_key_t* out_keys;       // [row_hi - row_lo, segments * parts, kLists, kTopK]; written when parts > 1, else null
     int* status;
     unsigned long long* stats; // cycle counters of a profiling build (-DVL_KNN_STATS), else unused
 };
@@ -222,6 +225,16 @@ __device__ __forceinline__ float min3f(float a, float b, float c)
     float r;
     asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
+}
+
+// candidates [c_begin, c_end) of candidate range `piece`: part piece % parts of segment piece / parts
+__device__ __forceinline__ void piece_range(const KnnArgs& a, int64_t piece, int64_t& c_begin, int64_t& c_end)
+{
+    const int64_t seg = piece / a.parts, part = piece % a.parts;
+    const int64_t s_begin = a.cand_lo + seg * a.seg_len;
+    const int64_t s_end = (s_begin + a.seg_len < a.cand_hi) ? s_begin + a.seg_len : a.cand_hi;
+    c_begin = s_begin + part * a.part_len;
+    c_end = (c_begin + a.part_len < s_end) ? c_begin + a.part_len : s_end;
 }
 
 // RESIDENT: the row tile (all its k-blocks) is loaded once per work item and only candidate
@@ -269,7 +282,8 @@ knn_tile_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
     const uint32_t tmem_base = *tmem_slot;
 
     const int64_t row_tiles = (a.row_hi - a.row_lo + kTileRows - 1) / kTileRows;
-    const int64_t items = row_tiles * a.segments;
+    const int64_t pieces = (int64_t)a.segments * a.parts;          // candidate ranges; `seg` below numbers them
+    const int64_t items = row_tiles * pieces;
 
     if (warp == 0 && lane == 0) {
         // ---------------- TMA producer ----------------
@@ -277,10 +291,10 @@ knn_tile_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         bool ok = true;
 #pragma unroll 1
         for (int64_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
-            const int64_t rt = item / a.segments, seg = item % a.segments;
+            const int64_t rt = item / pieces, seg = item % pieces;
             const int64_t row0 = a.row_lo + rt * kTileRows;
-            const int64_t c_begin = a.cand_lo + seg * a.seg_len;
-            const int64_t c_end = (c_begin + a.seg_len < a.cand_hi) ? c_begin + a.seg_len : a.cand_hi;
+            int64_t c_begin, c_end;
+            piece_range(a, seg, c_begin, c_end);
             if (RESIDENT && c_begin < c_end) {
                 // the previous item's MMAs must be done with the row tile before it is overwritten
                 ok = mbar_wait(bar_rows_empty, (nres & 1u) ^ 1u, abort_flag, a.status);
@@ -318,9 +332,9 @@ knn_tile_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         bool ok = true;
 #pragma unroll 1
         for (int64_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
-            const int64_t seg = item % a.segments;
-            const int64_t c_begin = a.cand_lo + seg * a.seg_len;
-            const int64_t c_end = (c_begin + a.seg_len < a.cand_hi) ? c_begin + a.seg_len : a.cand_hi;
+            const int64_t seg = item % pieces;
+            int64_t c_begin, c_end;
+            piece_range(a, seg, c_begin, c_end);
             if (RESIDENT && c_begin < c_end) {
                 ok = mbar_wait(bar_rows_full, nres & 1u, abort_flag, a.status);
                 if (!ok) break;
@@ -372,10 +386,10 @@ knn_tile_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         bool ok = true;
 #pragma unroll 1
         for (int64_t item = blockIdx.x; item < items && ok; item += gridDim.x) {
-            const int64_t rt = item / a.segments, seg = item % a.segments;
+            const int64_t rt = item / pieces, seg = item % pieces;
             const int64_t row = a.row_lo + rt * kTileRows + row_in_tile;
-            const int64_t c_begin = a.cand_lo + seg * a.seg_len;
-            const int64_t c_end = (c_begin + a.seg_len < a.cand_hi) ? c_begin + a.seg_len : a.cand_hi;
+            int64_t c_begin, c_end;
+            piece_range(a, seg, c_begin, c_end);
             // The kTopK best keys of each of this warp's 32 rows, ascending, in shared memory: row r's list is
             // warp_lists[r * kTopK + lane], one key per lane, so that an insertion is a warp-wide shift (a few
             // instructions) instead of a register sort by the one lane that owns the row.  Each lane keeps
@@ -518,8 +532,9 @@ knn_tile_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
                     const int r = r0 + lane / kTopK, kk = lane % kTopK;
                     if (first_row + r < a.row_hi) {
                         const vl_key_t k = warp_lists[r * kTopK + kk];
-                        a.out_ids[(((first_row + r - a.row_lo) * a.segments + seg) * kLists + cls) * kTopK + kk] =
-                            k == ~0ull ? VL_MAXINT : (int32_t)(uint32_t)k;
+                        const int64_t at = (((first_row + r - a.row_lo) * pieces + seg) * kLists + cls) * kTopK + kk;
+                        if (a.out_keys) a.out_keys[at] = k;
+                        else a.out_ids[at] = k == ~0ull ? VL_MAXINT : (int32_t)(uint32_t)k;
                     }
                 }
                 __syncwarp();
@@ -532,6 +547,36 @@ knn_tile_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant_
         __syncwarp();
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+    }
+}
+
+// The kTopK smallest keys of the `parts` ascending lists of one (row, segment, class), by one warp: lane p
+// walks list p, each round takes the smallest head.  Keys are distinct (they end in the candidate's id), so
+// the result is the list that one work item over the whole segment would have kept.
+__global__ void __launch_bounds__(256)
+knn_join_parts_kernel(const vl_key_t* __restrict__ keys, int64_t lists, int parts, int32_t* __restrict__ out_ids)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t l = warp0; l < lists; l += nwarps) {
+        const int64_t rs = l / kLists, cls = l % kLists;            // (row, segment), class
+        const vl_key_t* mine = keys + ((rs * parts + (lane < parts ? lane : 0)) * kLists + cls) * kTopK;
+        int next = 0;
+        vl_key_t head = lane < parts ? mine[0] : ~0ull;
+        int32_t got = VL_MAXINT;                                    // lane t keeps the t-th smallest
+        for (int t = 0; t < kTopK; ++t) {
+            const uint32_t hi = __reduce_min_sync(0xffffffffu, (uint32_t)(head >> 32));
+            const uint32_t lo = __reduce_min_sync(0xffffffffu, (uint32_t)(head >> 32) == hi ? (uint32_t)head : 0xffffffffu);
+            const vl_key_t best = ((vl_key_t)hi << 32) | lo;
+            if (best == ~0ull) break;
+            if (lane == t) got = (int32_t)lo;
+            if (head == best) {
+                ++next;
+                head = next < kTopK ? mine[next] : ~0ull;
+            }
+        }
+        if (lane < kTopK) out_ids[l * kTopK + lane] = got;
     }
 }
 
@@ -586,6 +631,14 @@ extern "C" int vl_knn_tile(const uint16_t* rows_bf16, int64_t n, int dim_pad, co
                            int64_t row_hi, int64_t cand_lo, int64_t cand_hi, int segments, int32_t* out_ids, int* status,
                            void* stream)
 {
+    return vl_knn_tile_parts(rows_bf16, n, dim_pad, sqnorm, row_lo, row_hi, cand_lo, cand_hi, segments, 1, nullptr, out_ids, status,
+                             stream);
+}
+
+extern "C" int vl_knn_tile_parts(const uint16_t* rows_bf16, int64_t n, int dim_pad, const float* sqnorm, int64_t row_lo,
+                                 int64_t row_hi, int64_t cand_lo, int64_t cand_hi, int segments, int parts,
+                                 unsigned long long* scratch, int32_t* out_ids, int* status, void* stream)
+{
     VL_CHECK_ARG(rows_bf16 && out_ids && status, "vl_knn_tile: null pointer");
     VL_CHECK_ARG(n > 0 && n < (1ll << 31), "vl_knn_tile: row count %lld outside int32", (long long)n);
     VL_CHECK_ARG(dim_pad > 0 && dim_pad % kBlockK == 0, "vl_knn_tile: padded dimension %d is not a multiple of %d", dim_pad, kBlockK);
@@ -593,6 +646,8 @@ extern "C" int vl_knn_tile(const uint16_t* rows_bf16, int64_t n, int dim_pad, co
     VL_CHECK_ARG(0 <= row_lo && row_lo <= row_hi && row_hi <= n, "vl_knn_tile: bad row range");
     VL_CHECK_ARG(0 <= cand_lo && cand_lo <= cand_hi && cand_hi <= n, "vl_knn_tile: bad candidate range");
     VL_CHECK_ARG(segments >= 1 && segments <= 64, "vl_knn_tile: segments %d outside 1..64", segments);
+    VL_CHECK_ARG(parts >= 1 && parts <= 32, "vl_knn_tile: parts %d outside 1..32", parts);
+    VL_CHECK_ARG(parts == 1 || scratch, "vl_knn_tile: parts need scratch");
     if (row_hi == row_lo) return 0;
 
     static EncodeTiledFn encode = nullptr;
@@ -630,7 +685,11 @@ extern "C" int vl_knn_tile(const uint16_t* rows_bf16, int64_t n, int dim_pad, co
     int64_t seg_len = (span + segments - 1) / segments;
     seg_len = (seg_len + kTileCands - 1) / kTileCands * kTileCands;
     a.seg_len = seg_len > 0 ? seg_len : kTileCands;
+    const int64_t part_len = (a.seg_len + parts - 1) / parts;
+    a.parts = parts;
+    a.part_len = (part_len + kTileCands - 1) / kTileCands * kTileCands;
     a.out_ids = out_ids;
+    a.out_keys = parts > 1 ? scratch : nullptr;
     a.status = status;
     a.stats = nullptr;
 #ifdef VL_KNN_STATS
@@ -641,10 +700,16 @@ extern "C" int vl_knn_tile(const uint16_t* rows_bf16, int64_t n, int dim_pad, co
     auto kernel = resident ? knn_tile_kernel<true> : knn_tile_kernel<false>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     VL_CHECK_ARG(e == cudaSuccess, "vl_knn_tile: %s", cudaGetErrorString(e));
-    const int64_t items = ((row_hi - row_lo + kTileRows - 1) / kTileRows) * segments;
+    const int64_t items = ((row_hi - row_lo + kTileRows - 1) / kTileRows) * segments * parts;
     const int sms = vl_sm_count();
     const unsigned grid = (unsigned)(items < sms ? items : sms);
     kernel<<<grid, kThreads, kSmemBytes, (cudaStream_t)stream>>>(tmap, tmap_cand, a);
     VL_CHECK_LAUNCH("knn_tile_kernel");
+    if (parts > 1) {
+        const int64_t lists = (row_hi - row_lo) * segments * kLists;
+        const int64_t blocks = (lists + 7) / 8, cap = (int64_t)sms * 16;
+        knn_join_parts_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, (cudaStream_t)stream>>>(scratch, lists, parts, out_ids);
+        VL_CHECK_LAUNCH("knn_join_parts_kernel");
+    }
     return 0;
 }
