@@ -55,6 +55,13 @@ int vl_search_from_seeds(const float* queries, int64_t b, const int32_t* visit, 
                          const float* vectors, int64_t n, int dim, int32_t* idx_out, float* dist_out, int metric,
                          int* status, void* stream);
 
+/* The seeds of a search (utils.py:26-32 + ann.py:217-232): idx_out[b, j] = (first_row + b + offsets[j]) mod
+ * modulo, in 32 bits, and dist_out[b, j] = distance(queries[b], vectors[idx_out[b, j]]); both [rows, w].
+ * 1 <= modulo <= n. */
+int vl_circulant_seeds(const float* vectors, int64_t n, int dim, const float* queries, int64_t rows,
+                       const int32_t* offsets, int w, int64_t first_row, int64_t modulo, int32_t* idx_out,
+                       float* dist_out, int metric, int* status, void* stream);
+
 /* Queue.insert (queue.py:37-61): rows [b, cap] of ids/dist in place.  The m candidates go to
  * columns [length, length+m), ids found in the row's exclusion list excl[b, 0..e) (scanned up
  * to its first MAXINT; kernels.py:471-488) become sentinels, then the whole row is ordered by

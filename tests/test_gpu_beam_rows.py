@@ -143,3 +143,18 @@ def test_divided_segments_give_the_same_proposals(rows, cands, segments, parts, 
     finally:
         knn_tile._parts = keep
     assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("metric", ["cosine", "l2"])
+@pytest.mark.parametrize("dim", [1, 50, 64, 96, 128, 250, 256, 384, 512, 768, 1024, 1030])
+def test_circulant_seeds_equal_the_operators(dim, metric, built_lib):
+    """Seed ids and distances of one kernel against the two operators, rows and widths off every step and run size."""
+    from vectorlink_gpu.kernels import calculate_distances, circulant_seeds
+    from vectorlink_gpu.utils import generate_queue_circulants, primes, seed_offsets
+    vectors = rows_of(9, 701, dim, metric)
+    for (rows, w, first_row, modulo) in ((1, 1, 0, 701), (1, 64, 5, 701), (3, 1920, 0, 701), (157, 33, 10_000, 700), (5000, 31, 0, 1)):
+        queries = rows_of(10, rows, dim, metric)
+        ids = generate_queue_circulants(rows, modulo, primes(w, DEV), first_row)
+        want = calculate_distances(vectors, ids, metric=metric, queries=queries)
+        (got_ids, got) = circulant_seeds(vectors, queries, seed_offsets(w, DEV), first_row, modulo, metric)
+        assert torch.equal(got_ids, ids) and torch.equal(got, want)

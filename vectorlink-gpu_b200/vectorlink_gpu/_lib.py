@@ -20,7 +20,7 @@ c_u32p = ctypes.POINTER(ctypes.c_uint32)
 c_intp = ctypes.POINTER(ctypes.c_int)
 
 EXPORTS = [
-    "vl_last_error", "vl_abi_version", "vl_calculate_distances", "vl_search_from_seeds", "vl_queue_insert",
+    "vl_last_error", "vl_abi_version", "vl_calculate_distances", "vl_circulant_seeds", "vl_search_from_seeds", "vl_queue_insert",
     "vl_queue_pop", "vl_punchout_excluded", "vl_dedup_adjacent", "vl_sort_pairs", "vl_dedup_sort_ids",
     "vl_seen_add", "vl_seen_add_noalloc", "vl_prune", "vl_prune_rows", "vl_reverse_edges", "vl_connected_components", "vl_beam_search",
     "vl_beam_search_rows", "vl_beam_search_plan", "vl_locality_keys", "vl_knn_prepare", "vl_knn_tile", "vl_knn_tile_parts",
@@ -69,6 +69,7 @@ def lib() -> ctypes.CDLL:
             getattr(_lib, name).restype = ctypes.c_int
         P, I, L = ctypes.c_void_p, ctypes.c_int, ctypes.c_int64
         _lib.vl_calculate_distances.argtypes = [P, L, I, P, L, P, I, P, I, P, P]
+        _lib.vl_circulant_seeds.argtypes = [P, L, I, P, L, P, I, L, L, P, P, I, P, P]
         _lib.vl_search_from_seeds.argtypes = [P, L, P, I, P, I, P, L, I, P, P, I, P, P]
         _lib.vl_queue_insert.argtypes = [P, P, L, I, I, P, P, I, P, I, P, P]
         _lib.vl_queue_pop.argtypes = [P, P, L, I, I, I, P, P]

@@ -18,12 +18,12 @@ from torch import Tensor
 
 from . import _lib
 from ._lib import BeamParams, check, lib, ptr, stream_of
-from .constants import MAXFLOAT, MAXINT, PRIMES_HOST
-from .kernels import calculate_distances, connected_components, metric_code, prune_, search_from_seeds, sort_pairs_
+from .constants import DEBUG, MAXFLOAT, MAXINT, PRIMES_HOST
+from .kernels import calculate_distances, circulant_seeds, connected_components, metric_code, prune_, search_from_seeds, sort_pairs_
 from .log import log_time, nvtx_range
 from . import log as _log
 from .queue import Queue
-from .utils import add_new_to_seen_, generate_circulant_beams, generate_queue_circulants, primes
+from .utils import add_new_to_seen_, generate_circulant_beams, generate_queue_circulants, primes, seed_offsets
 
 FUSED_MAX_SMEM_PER_ROW = 200 * 1024
 # When set to a list, every fused-kernel launch appends its CUDA events (recorded on the
@@ -120,14 +120,15 @@ def _launch_beam(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_len
     p.memo_slots = 0
     p.stats = stats.data_ptr() if stats is not None else 0
     p.flags = 0
+    smem, per_block, blocks = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
+    check(lib().vl_beam_search_plan(ctypes.byref(p), ctypes.byref(smem), ctypes.byref(per_block), ctypes.byref(blocks)),
+          "vl_beam_search_plan")
+    scratch = blocks.value > 0          # else every row is in flight at once with its memo on chip
     # rows differ in the work they take: CTAs draw their next row from a counter instead of a fixed stride
-    ticket = torch.zeros(1, dtype=torch.int64, device=vectors.device) if config.get("row_ticket", True) else None
+    ticket = torch.zeros(1, dtype=torch.int64, device=vectors.device) if scratch and config.get("row_ticket", True) else None
     p.row_ticket = ticket.data_ptr() if ticket is not None else 0
-    if config.get("memo", True):
+    if scratch and config.get("memo", True):
         # id -> distance memo of each row in flight (scratch; the kernel clears a row's slice)
-        smem, per_block, blocks = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
-        check(lib().vl_beam_search_plan(ctypes.byref(p), ctypes.byref(smem), ctypes.byref(per_block), ctypes.byref(blocks)),
-              "vl_beam_search_plan")
         entries = int(config.get("memo_entries", 0))
         if entries <= 0:
             entries = 1024        # measured on 1M x 128: 8192 entries per row at E=320 (24*E) is the knee
@@ -362,6 +363,27 @@ def closest_vectors(query_vecs: Tensor, search_queue: Queue, vectors: Tensor, be
 closest_vectors.last_count = 0
 
 
+def _seeded_search(query: Tensor, seeds: Tensor, seed_dist: Tensor, vectors: Tensor, beams: Tensor, config: Dict,
+                   queue_size: int, queue_capacity: int, seeded_queue) -> Queue:
+    """Search of every query row from an empty queue and its seeds, which the fused kernel inserts itself: no
+    separate sort, and no queue to fill first (the kernel writes every column).  `seeded_queue()`: the queue
+    with the seeds inserted, for a batch that the operator path has to take."""
+    rows = query.size(0)
+    queue = Queue.uninitialized(rows, queue_size, queue_capacity, device=vectors.device)
+
+    def stepwise(lo, hi):
+        q = seeded_queue()
+        n = closest_vectors_stepwise(query, q, vectors, beams, config, None)
+        queue.indices.copy_(q.indices)
+        queue.distances.copy_(q.distances)
+        return n
+
+    counts = _fused_batches(vectors, beams, query, seeds, seed_dist, seeds.size(1), queue_size, queue_capacity, config, None, -1,
+                            rows, queue.indices, queue.distances, queue_capacity, stepwise)
+    closest_vectors.last_count = counts[0]
+    return queue
+
+
 def search_layers(layers: List[Tensor], query_vecs: Tensor, search_queue: Queue, vectors: Tensor, config: Dict):
     """ann.py:96-106."""
     for layer in layers:
@@ -550,6 +572,21 @@ def initial_queue(vectors: Tensor, config: Dict):
     return queue
 
 
+def _self_search(sample: Tensor, vectors: Tensor, beams: Tensor, config: Dict) -> Queue:
+    """The search queues of the first rows of `vectors` (`sample`), from circulant seeds among themselves."""
+    (rows, _) = sample.size()
+    queue_size = config["recall_search_queue_factor"] * config["beam_size"]
+    capacity = queue_size + max(queue_size, config["parallel_visit_count"] * config["beam_size"])
+    if rows == 0 or DEBUG or config.get("stepwise", False) or not _fused_queue_ok(beams.size(1), queue_size, capacity, config):
+        queue = initial_queue(sample, config)
+        closest_vectors(sample, queue, vectors, beams, config)
+        return queue
+    _lib.require_cuda(sample, vectors, beams)
+    assert vectors.is_contiguous() and beams.is_contiguous()
+    (seeds, d) = circulant_seeds(sample, sample, seed_offsets(queue_size, vectors.device), 0, rows, _metric_of(config))
+    return _seeded_search(sample, seeds, d, vectors, beams, config, queue_size, capacity, lambda: initial_queue(sample, config))
+
+
 def query_distances(query_vectors: Tensor, vectors: Tensor, ids: Tensor, metric="cosine") -> Tensor:
     """Distances of query b to vectors[ids[b, j]] (the role of query_cosine_distances,
     ann.py:211-214, whose broadcast only works for one query row).  Taken with the same
@@ -589,8 +626,7 @@ def ann_calculate_recall(vectors: Tensor, beams: Tensor, config: Dict, sample: O
     if sample is None:
         sample = vectors
     (sample_size, _) = sample.size()
-    queue = initial_queue(sample.contiguous(), config)
-    closest_vectors(sample.contiguous(), queue, vectors, beams.contiguous(), config)
+    queue = _self_search(sample.contiguous(), vectors, beams.contiguous(), config)
     expected = torch.arange(sample_size, device=vectors.device)
     actual = queue.indices.t()[0]
     found = (expected == actual).sum().item()
@@ -784,9 +820,7 @@ class ANN:
         """ann.py:466-467 is an empty stub; its README says it "returns all search queues":
         the search queue of every indexed vector, seeded like the recall check
         (initial_queue) and searched through the graph."""
-        queue = initial_queue(self.vectors, self.configuration)
-        closest_vectors(self.vectors, queue, self.vectors, self.beams, self.configuration)
-        return queue
+        return _self_search(self.vectors, self.vectors, self.beams.contiguous(), self.configuration)
 
     def cluster_labels(self, threshold: float, queues: Optional[Queue] = None) -> Tensor:
         """Clusters as connected components (added; the reference stops at the `clusters` stub):
@@ -834,28 +868,14 @@ class ANN:
                 closest_vectors(query, search_queue, self.vectors, beams, config, None)
                 return search_queue
             seed_count = seeds.size(1)
-        if (entry_sample > 0 or seed_count > extra_capacity) and fused_ok:
-            # many seeds: the fused kernel starts every row from an empty queue and merges the
-            # seeds itself, so the best-Q selection needs no separate sort
+        # (with DEBUG the search proper is timed as one call of closest_vectors, so it gets its queue ready-made)
+        if fused_ok and (entry_sample > 0 or seed_count > extra_capacity or not DEBUG):
             _lib.require_cuda(query, self.vectors, beams)
-            dev = self.vectors.device
             if entry_sample <= 0:
-                seeds = generate_queue_circulants(query.size(0), self.vectors.size(0), primes(seed_count, dev), first_row)
-                d = query_distances(query, self.vectors, seeds, _metric_of(config))
-            queue = Queue(query.size(0), queue_size, queue_size + extra_capacity, device=dev)
-
-            def stepwise(lo, hi):
-                q = seeded_queue() if entry_sample > 0 else initial_search_queue(self.vectors, query, config, first_row)
-                n = closest_vectors_stepwise(query, q, self.vectors, beams, config, None)
-                queue.indices.copy_(q.indices)
-                queue.distances.copy_(q.distances)
-                return n
-
-            counts = _fused_batches(self.vectors, beams, query, seeds, d, seed_count, queue_size,
-                                    queue_size + extra_capacity, config, None, -1, query.size(0), queue.indices,
-                                    queue.distances, queue_size + extra_capacity, stepwise)
-            closest_vectors.last_count = counts[0]
-            return queue
+                (seeds, d) = circulant_seeds(self.vectors, query, seed_offsets(seed_count, self.vectors.device), first_row,
+                                             self.vectors.size(0), _metric_of(config))
+                seeded_queue = lambda: initial_search_queue(self.vectors, query, config, first_row)  # noqa: E731
+            return _seeded_search(query, seeds, d, self.vectors, beams, config, queue_size, queue_size + extra_capacity, seeded_queue)
         search_queue = initial_search_queue(self.vectors, query, config, first_row)
         closest_vectors(query, search_queue, self.vectors, beams, config, None)
         return search_queue

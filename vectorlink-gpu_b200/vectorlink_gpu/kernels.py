@@ -56,6 +56,24 @@ def calculate_distances(vectors: Tensor, beams: Tensor, distances_out=None, metr
     return distances_out
 
 
+def circulant_seeds(vectors: Tensor, queries: Tensor, offsets: Tensor, first_row: int, modulo: int,
+                    metric="cosine") -> Tuple[Tensor, Tensor]:
+    """utils.generate_queue_circulants and the distances of those ids in one kernel: ids[b, j] =
+    (first_row + b + offsets[j]) mod modulo, dist[b, j] = distance(queries[b], vectors[ids[b, j]])."""
+    assert vectors.dtype == torch.float32 and vectors.is_contiguous()
+    assert queries.dtype == torch.float32 and queries.is_contiguous() and queries.size(1) == vectors.size(1)
+    assert offsets.dtype == torch.int32 and offsets.is_contiguous()
+    _lib.require_cuda(vectors, queries, offsets)
+    (rows, w) = (queries.size(0), offsets.size(0))
+    ids = torch.empty((rows, w), dtype=torch.int32, device=vectors.device)
+    dist = torch.empty((rows, w), dtype=torch.float32, device=vectors.device)
+    check(lib().vl_circulant_seeds(ptr(vectors), ctypes.c_int64(vectors.size(0)), vectors.size(1), ptr(queries),
+                                   ctypes.c_int64(rows), ptr(offsets), w, ctypes.c_int64(first_row), ctypes.c_int64(modulo),
+                                   ptr(ids), ptr(dist), metric_code(metric), ptr(_lib.status_word(vectors.device)),
+                                   stream_of(vectors)), "vl_circulant_seeds")
+    return ids, dist
+
+
 def search_from_seeds(query_vecs: Tensor, neighbors_to_visit: Tensor, beams: Tensor, vectors: Tensor,
                       metric="cosine") -> Tuple[Tensor, Tensor]:
     """kernels.py:260-311: ids and distances of the neighbours of the visited nodes, slot

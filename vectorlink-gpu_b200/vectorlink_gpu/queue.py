@@ -24,6 +24,16 @@ class Queue:
         self.indices = torch.full((num_queues, capacity), MAXINT, dtype=torch.int32, device=device)
         self.distances = torch.full((num_queues, capacity), MAXFLOAT, dtype=torch.float32, device=device)
 
+    @classmethod
+    def uninitialized(cls, num_queues: int, queue_length: int, capacity: int, device="cuda") -> "Queue":
+        """A queue whose columns the caller writes, all of them."""
+        assert queue_length < capacity
+        queue = cls.__new__(cls)
+        queue.length = queue_length
+        queue.indices = torch.empty((num_queues, capacity), dtype=torch.int32, device=device)
+        queue.distances = torch.empty((num_queues, capacity), dtype=torch.float32, device=device)
+        return queue
+
     def initialize_from_queue(self, queue: "Queue"):
         """queue.py:30-35."""
         head_length = min(queue.length, self.length)

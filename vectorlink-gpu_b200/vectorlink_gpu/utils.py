@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional
 
 import torch
@@ -30,6 +31,18 @@ def primes(size: int, device="cuda") -> Tensor:
     ext = (table.long()[j % table.numel()] * (j // table.numel() + 1) + j) % (1 << 30)
     ext[: table.numel()] = table.long()
     return ext.to(torch.int32)
+
+
+@functools.lru_cache(maxsize=64)
+def _sorted_primes(size: int, device: torch.device) -> Tensor:
+    out = primes(size, device).sort().values
+    torch.cuda.current_stream(device).synchronize()     # complete before a caller on another stream meets it
+    return out
+
+
+def seed_offsets(size: int, device) -> Tensor:
+    """The first `size` seed offsets in rising order: a constant table, kept per size and device."""
+    return _sorted_primes(size, _lib._device_key(device))
 
 
 def generate_queue_circulants(batch_size: int, num_vecs: int, primes: Tensor, first_row: int = 0) -> Tensor:
