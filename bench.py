@@ -285,7 +285,7 @@ def roofline_of(build_classes, search_classes, peak, peak_kind, workload, dim, k
         classes[cls] = entry
     head = classes.get("build_later_rounds") or classes.get("build_round0") or {}
     served = "DRAM" if "build_later_rounds" in classes else "mostly L2 (single-round build: circulant band)"
-    return {"bound": "hbm", "kernel": "beam_search_kernel", "class": "build_later_rounds" if "build_later_rounds" in classes else "build_round0",
+    return {"bound": "hbm", "kernel": "beam_team_kernel", "class": "build_later_rounds" if "build_later_rounds" in classes else "build_round0",
             "achieved": head.get("gathered_gbs"), "peak": peak, "unit": "GB/s",
             "frac": (head.get("gathered_gbs") or 0.0) / peak, "peak_source": peak_kind,
             "frac_of_8TBs_nominal": (head.get("gathered_gbs") or 0.0) / 8000.0,
