@@ -253,7 +253,7 @@ int vl_locality_keys(const int32_t* graph, int64_t n, int w, int64_t row_lo, int
 
 /* Bytes of shared memory one query row in flight of vl_beam_search needs for the given shape, the rows
  * per CTA and the CTAs it will launch.  blocks * rows_per_block is the number of rows in flight, i.e.
- * the memo_slots a distance memo must provide; 0 blocks: the rows keep their memo on chip and the launch
+ * the memo_slots a distance memo must provide (it depends on memo_entries; memo may still be NULL); 0 blocks: the rows keep their memo on chip and the launch
  * needs no scratch.
  *
  * The memo: during one row's search the same candidate id comes back many times (neighbour

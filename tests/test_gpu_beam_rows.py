@@ -27,8 +27,8 @@ def search_both_ways(ann, queries):
     return out
 
 
-# one row per SM (16 or 8 warps), two (8), four (4), eight (2), more (two warps, memo in global memory); 148 SMs
-@pytest.mark.parametrize("count", [1, 2, 5, 148, 149, 296, 297, 592, 593, 1184, 1185, 2500])
+# one row per SM (16 or 8 warps), two (8), four (4), eight (2), more (one or two warps, memo in global memory); 148 SMs
+@pytest.mark.parametrize("count", [1, 2, 5, 148, 149, 296, 297, 592, 593, 1184, 1185, 3100])
 @pytest.mark.parametrize("metric,dim,degree", [("cosine", 64, 16), ("l2", 100, 24), ("cosine", 768, 64)])
 def test_every_split_of_a_row_gives_the_operator_path_queues(count, metric, dim, degree, built_lib):
     from vectorlink_gpu import ANN, _lib
@@ -40,6 +40,17 @@ def test_every_split_of_a_row_gives_the_operator_path_queues(count, metric, dim,
     assert torch.equal(fused[0], steps[0]) and torch.equal(fused[1], steps[1])
     assert fused[2] == steps[2]
     assert _lib.read_status(DEV) == 0
+
+
+@pytest.mark.parametrize("count", [2369, 2960, 2961])      # around one wave of either split at 256 dimensions
+@pytest.mark.parametrize("memo", [{}, {"memo": False}, {"memo_entries": 2}, {"memo_entries": 4096}, {"memo_entries": 8192}])
+def test_one_or_two_warps_per_row_give_the_same_queues(count, memo, built_lib):
+    from vectorlink_gpu import ANN
+    ann = ANN(vectors=rows_of(1, 3001, 256, "l2"), beam_size=8, visit_queue_factor=2, recall_search_queue_factor=2,
+              metric="l2", init="knn_tile", optimization_loops=1)
+    ann.configuration.update(memo)
+    (fused, steps) = search_both_ways(ann, rows_of(2, count, 256, "l2"))
+    assert torch.equal(fused[0], steps[0]) and torch.equal(fused[1], steps[1]) and fused[2] == steps[2]
 
 
 def test_a_batch_that_stops_early_ends_together(built_lib):

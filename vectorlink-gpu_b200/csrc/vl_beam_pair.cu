@@ -1,4 +1,5 @@
-// Fused beam search with two warps per query row, 16 rows in flight per SM: launches of many rows.
+// Fused beam search with two warps per query row and 16 rows in flight per SM, or one warp and 20 rows:
+// launches of many rows.
 //
 // A row's iteration is a chain of memory round trips and queue steps, so a launch is bound by latency
 // at the number of rows that can be in flight.  That number is bound in turn by the rows' memos
@@ -12,14 +13,20 @@
 // 10,000 searches of 1,000,000 x 128: 6.6 / 5.3; 2,500 of 200,000 x 256: 2.33 / 1.55.  12 rows per SM at 80
 // registers (two gather steps in flight): 541, 119, 81; one warp per row with the same queue step at 16 rows per
 // SM: 528, 137, 75, at 24 rows per SM: 740, 144, 108.
+//
+// One warp per row and 20 rows per SM (vl_beam_solo) is better where a row's memo is small (32 KB or none, so that
+// 2,960 of them do not push each other out of L2) and its rows are short: searches of 30,000 x 96 (clusters)
+// 10.0 / 8.9 ms, 10,000 of 1,000,000 x 128 5.2 / 4.8, the first build round (no memo) of 150,000 x 128 253 / 227.  Rows
+// of 256 dimensions gain only where 20 rows per SM save a wave (2,500 searches: 1.54 / 1.08; first round of
+// 20,000: 44.8 / 46.9); 768 dimensions lose (3,000 searches: 3.3 / 4.9).
 #include "vl_beam_team.cuh"
 
 namespace {
 
-template <int LPR, int JP, int JU, int METRIC, bool ALIGNED>
-int pair_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)
+template <int TEAM, int LPR, int JP, int JU, int METRIC, bool ALIGNED>
+int many_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)
 {
-    auto kernel = beam_team_kernel<LPR, JP, JU, METRIC, ALIGNED, 2>;
+    auto kernel = beam_team_kernel<LPR, JP, JU, METRIC, ALIGNED, TEAM>;
     const TeamSmem lay = team_layout(p.pvc * p.graph_w, p.sq_len, p.vq_len, p.seen_cap, LPR * JP * 16, p.memo ? p.memo_entries : 0, false);
     int dev = 0, max_smem = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -28,7 +35,7 @@ int pair_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, 
     VL_CHECK_ARG(lay.total <= max_smem, "vl_beam_search: one row needs %d bytes of shared memory, the device offers %d", lay.total, max_smem);
     e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lay.total);
     VL_CHECK_ARG(e == cudaSuccess, "vl_beam_search: %s", cudaGetErrorString(e));
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 64, lay.total);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * TEAM, lay.total);
     VL_CHECK_ARG(e == cudaSuccess && per_sm > 0, "vl_beam_search: occupancy query failed");
     const int64_t resident = (int64_t)vl_sm_count() * per_sm;   // one resident wave; further rows are drawn as CTAs finish
     const int grid = (int)(p.rows < resident ? p.rows : resident);
@@ -37,9 +44,27 @@ int pair_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, 
     if (!launch) return 0;
     VL_CHECK_ARG(!p.memo || p.memo_slots >= grid, "vl_beam_search: memo has %lld slots, the launch keeps %d rows in flight",
                  (long long)p.memo_slots, grid);
-    kernel<<<grid, 64, lay.total, stream>>>(p, lay, row_order, nullptr);
+    kernel<<<grid, 32 * TEAM, lay.total, stream>>>(p, lay, row_order, nullptr);
     VL_CHECK_LAUNCH("beam_team_kernel");
     return 0;
+}
+
+// the choice described above
+bool vl_beam_solo(const vl_beam_params& p)
+{
+    if (p.dim > 256 || p.memo_entries > 4096) return false;
+    if (p.dim <= 128) return true;
+    const int64_t sms = vl_sm_count();
+    return p.rows > sms * many_per_sm(2) && p.rows <= sms * many_per_sm(1);
+}
+
+template <int LPR, int JP, int JU, int METRIC, bool ALIGNED>
+int pair_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)
+{
+    if constexpr (LPR * JP <= 64) {     // 256 dimensions
+        if (vl_beam_solo(p)) return many_launch<1, LPR, JP, JU, METRIC, ALIGNED>(p, row_order, launch, blocks, smem, stream);
+    }
+    return many_launch<2, LPR, JP, JU, METRIC, ALIGNED>(p, row_order, launch, blocks, smem, stream);
 }
 
 }  // namespace

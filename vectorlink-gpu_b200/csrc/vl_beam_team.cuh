@@ -2,14 +2,16 @@
 //
 // An iteration of a row is: neighbour ids and memo probes, the gather of the candidates the memo does not
 // know, the choice of those that can enter a queue - each split over all warps - and then the two
-// queue steps side by side, the search queue's on warp 0 and the visit queue's on warp 1.
+// queue steps, side by side where there are warps for it (the search queue's on warp 0, the visit queue's
+// on warp 1).
 #pragma once
 #include "vl_beam.cuh"
 
 namespace {
 
 constexpr int kMaxTeam = 16;                                   // most warps per row
-constexpr int kPairsPerSm = 16;                                // rows in flight per SM that teams of two aim for
+// CTAs per SM that launches of many rows aim for: teams of one warp (96 registers) or two (64)
+constexpr int many_per_sm(int team) { return team == 1 ? 20 : 16; }
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;     // 2 s per wait
 
 struct TeamSmem {      // carve-up of the CTA's shared memory, in bytes
@@ -169,7 +171,7 @@ __device__ __forceinline__ void team_gather(const vl_beam_params& p, uint2* cand
 {
     constexpr int G = 32 / LPR;
     constexpr int JX = JU > 0 ? JU : JP;
-    constexpr int U = TEAM == 2 ? 1 : (JU > 0 ? (JX <= 4 ? 4 : 2) : 1);
+    constexpr int U = TEAM == 1 ? (JX <= 4 ? 2 : 1) : TEAM == 2 ? 1 : (JU > 0 ? (JX <= 4 ? 4 : 2) : 1);
     const int g = lane / LPR, lg = lane % LPR;
 #pragma unroll 1
     for (int t0 = warp * G; t0 < n; t0 += nwarps * U * G) {
@@ -185,7 +187,7 @@ __device__ __forceinline__ void team_gather(const vl_beam_params& p, uint2* cand
             const int32_t id = live[u] ? (int32_t)cand[mi[u]].x : 0;
             rp[u] = p.vectors + (int64_t)id * p.dim;
         }
-        if constexpr (JU > 0 && TEAM == 2) {
+        if constexpr (JU > 0 && TEAM <= 2) {
             // pull the next round of candidate rows into L1 while this one is reduced
             constexpr int LINES = (4 * LPR * JU * 4) / 128;          // 128-byte lines per row
             const int tn = t0 + nwarps * U * G;
@@ -224,17 +226,17 @@ __device__ __forceinline__ void team_gather(const vl_beam_params& p, uint2* cand
     }
 }
 
-// TEAM == 2: launches of many rows, kPairsPerSm CTAs per SM, the memo in global memory (L2).
+// TEAM <= 2: launches of many rows, many_per_sm(TEAM) CTAs per SM, the memo in global memory (L2).
 // TEAM == kMaxTeam: launches of few rows, 2 to 16 warps per CTA (blockDim), the memo in shared memory.
 // JU > 0: exact-fit rows (dim == 4*LPR*JU, see vl_load_exact); JU == 0: any dimension, with 128-bit
 // loads when ALIGNED (dim % 4 == 0 and 16-byte aligned rows) and four scalar loads per chunk otherwise.
 template <int LPR, int JP, int JU, int METRIC, bool ALIGNED, int TEAM>
-__global__ void __launch_bounds__(TEAM * 32, TEAM == 2 ? kPairsPerSm : 1)
+__global__ void __launch_bounds__(TEAM * 32, TEAM <= 2 ? many_per_sm(TEAM) : 1)
 beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __restrict__ row_order, unsigned int* arrivals)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, threads = TEAM == 2 ? 64 : blockDim.x, nwarps = threads >> 5;
-    vl_key_t* memo = TEAM == 2 ? (p.memo ? p.memo + (size_t)blockIdx.x * (size_t)p.memo_entries : nullptr)
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, threads = TEAM <= 2 ? TEAM * 32 : blockDim.x, nwarps = threads >> 5;
+    vl_key_t* memo = TEAM <= 2 ? (p.memo ? p.memo + (size_t)blockIdx.x * (size_t)p.memo_entries : nullptr)
                                : reinterpret_cast<vl_key_t*>(smem + lay.memo);
     float4* q4 = reinterpret_cast<float4*>(smem + lay.query);
     uint2* cand = reinterpret_cast<uint2*>(smem + lay.cand);
@@ -255,8 +257,8 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
     const float inv_wb = 1.0f / (float)wb;
     // With a memo a candidate row is read about once per query row: unless rows are taken neighbourhood by
     // neighbourhood, stream it through L2 and keep the graph rows and the memo there instead.
-    const uint64_t pol_stream = (TEAM == 2 && p.memo && !row_order) ? vl_policy_evict_first() : vl_policy_evict_normal();
-    const uint64_t pol_keep = (TEAM == 2 && p.memo) ? vl_policy_evict_last() : vl_policy_evict_normal();
+    const uint64_t pol_stream = (TEAM <= 2 && p.memo && !row_order) ? vl_policy_evict_first() : vl_policy_evict_normal();
+    const uint64_t pol_keep = (TEAM <= 2 && p.memo) ? vl_policy_evict_last() : vl_policy_evict_normal();
 
     // Row schedule: the first row of a CTA is fixed; after that either a fixed stride or, when the caller
     // provides a zeroed counter, the next row nobody has taken yet (rows take unequal time).  `place`
@@ -358,7 +360,7 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
             if (__any_sync(0xffffffffu, lane < ncopy && popped == VL_MAXINT)) always_full = false;
             // ---- neighbour ids (kernels.py:244), then which of them need a gather: live ids the memo does not know.
             // PB chunks per warp and round: the graph-row loads, then the memo loads, of a round are in flight together.
-            constexpr int PB = TEAM == 2 ? 6 : 4;
+            constexpr int PB = TEAM <= 2 ? 6 : 4;
 #pragma unroll 1
             for (int cb = warp * 32; cb < m_total; cb += threads * PB) {
                 int32_t idr[PB];
@@ -379,7 +381,7 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
                     bk[u] = make_ulonglong2(~0ull, ~0ull);
                     if (memo && idr[u] != VL_MAXINT) {
                         const ulonglong2* at = reinterpret_cast<const ulonglong2*>(memo) + memo_bucket((uint32_t)idr[u], lay.memo_shift, lay.memo_buckets);
-                        if constexpr (TEAM == 2) bk[u] = vl_ld_hint(at, pol_keep);
+                        if constexpr (TEAM <= 2) bk[u] = vl_ld_hint(at, pol_keep);
                         else bk[u] = *at;
                     }
                 }
@@ -470,7 +472,7 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
                     if ((k % p.readahead) == 0 && chk < p.n_checks) {
                         unsigned int* flag = p.changed_flags + group * p.n_checks + chk;
                         if (changed) atomicOr(flag, 1u);
-                        if (TEAM != 2 && arrivals) {
+                        if (TEAM > 2 && arrivals) {
                             __threadfence();
                             atomicAdd(arrivals + chk, 1u);
                             if (!changed && waits) {
@@ -495,7 +497,8 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
                         }
                     }
                 }
-            } else if (warp == 1) {
+            }
+            if (warp == (TEAM == 1 ? 0 : 1)) {
                 // ---- the popped heads leave, visit_queue.insert(..., exclude=seen) ----
                 vl_key_t* vq_n = reinterpret_cast<vl_key_t*>(smem + (lay.vq_a + lay.vq_b - ctl[kVqBuf]));
                 const int n_a = usual ? ctl[kListV] : (seen_live ? m_total : 0);   // an (almost) empty queue is offered every candidate
@@ -548,7 +551,7 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
                 mark_popped(vq, k + 1);
             }
             __syncthreads();
-            if (TEAM != 2 && ctl[kStop] != 0) {
+            if (TEAM > 2 && ctl[kStop] != 0) {
                 // The batch ends here: this iteration's insert is left to the caller's full-row sort, which
                 // wants every candidate's distance; those of visited ids are taken again.
 #pragma unroll 1
@@ -587,7 +590,8 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
                 atomicAdd(p.stats + 2, (unsigned long long)st_m);
                 atomicAdd(p.stats + 6, 1ull);
                 atomicAdd(p.stats + 7, (unsigned long long)(k <= n_run ? k : n_run));
-            } else if (warp == 1) {
+            }
+            if (warp == (TEAM == 1 ? 0 : 1)) {
                 atomicAdd(p.stats + 3, (unsigned long long)st_v);
                 atomicAdd(p.stats + 4, (unsigned long long)st_a);
                 atomicAdd(p.stats + 5, (unsigned long long)st_b);

@@ -116,10 +116,10 @@ def _launch_beam(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_len
     p.group_full = full.data_ptr()
     p.status = _lib.status_word(vectors.device).data_ptr()
     p.memo = 0
-    p.memo_entries = 0
     p.memo_slots = 0
     p.stats = stats.data_ptr() if stats is not None else 0
     p.flags = 0
+    p.memo_entries = _memo_entries(p, config)
     smem, per_block, blocks = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
     check(lib().vl_beam_search_plan(ctypes.byref(p), ctypes.byref(smem), ctypes.byref(per_block), ctypes.byref(blocks)),
           "vl_beam_search_plan")
@@ -127,17 +127,11 @@ def _launch_beam(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_len
     # rows differ in the work they take: CTAs draw their next row from a counter instead of a fixed stride
     ticket = torch.zeros(1, dtype=torch.int64, device=vectors.device) if scratch and config.get("row_ticket", True) else None
     p.row_ticket = ticket.data_ptr() if ticket is not None else 0
-    if scratch and config.get("memo", True):
+    if scratch and p.memo_entries:
         # id -> distance memo of each row in flight (scratch; the kernel clears a row's slice)
-        entries = int(config.get("memo_entries", 0))
-        if entries <= 0:
-            entries = 1024        # measured on 1M x 128: 8192 entries per row at E=320 (24*E) is the knee
-            while entries < 24 * p.seen_cap and entries < 16384:
-                entries *= 2
         slots = max(1, per_block.value * blocks.value)
-        memo = _memo_buffer(vectors.device, slots * entries)
+        memo = _memo_buffer(vectors.device, slots * p.memo_entries)
         p.memo = memo.data_ptr()
-        p.memo_entries = entries
         p.memo_slots = slots
     order = _row_order(graph, self_base, queries.size(0), config) if p.memo else None
     if PROFILE is not None:
@@ -169,6 +163,23 @@ def _row_order(graph: Tensor, self_base: int, rows: int, config: Dict) -> Option
     check(lib().vl_locality_keys(ptr(graph), ctypes.c_int64(n), w, ctypes.c_int64(self_base),
                                  ctypes.c_int64(self_base + rows), ptr(near), ptr(keys), stream_of(graph)), "vl_locality_keys")
     return torch.argsort(keys)
+
+
+def _memo_entries(p: BeamParams, config: Dict) -> int:
+    """Entries of a row's distance memo: a row gathers about a quarter of the neighbours it looks at, and the
+    memos of the rows in flight share L2.  Measured: 8,192 is the knee of a 1M x 128 build (E = 320, lists
+    of 96); a search looks at a third of that, and 4,096 instead of 8,192 or 16,384 entries make searches of 96 and
+    128 dimensions 2-8 % faster, while on wider rows the gathers it repeats cost more (768 dimensions: 9 %
+    slower), so those get twice as many."""
+    if not config.get("memo", True):
+        return 0
+    entries = int(config.get("memo_entries", 0))
+    if entries <= 0:
+        need = min(24 * p.seen_cap, p.seen_cap * p.graph_w // (4 if p.dim <= 128 else 2))
+        entries = 1024
+        while entries < need and entries < 16384:
+            entries *= 2
+    return entries
 
 
 _memo_cache = {}
