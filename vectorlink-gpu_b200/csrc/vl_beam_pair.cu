@@ -6,7 +6,7 @@
 // (64 KB each at a build's 30,720 evaluations, 155 MB in all, already more than the 126 MB L2), not by
 // registers: a second warp per row halves the id, memo and gather phases and runs the two queue steps side
 // by side at 64 registers per thread, without another row's memo.  Build rounds, ms, one warp per row with
-// the queue merges of before (128 registers) / this, on one B200:
+// the queue merges of before (128 registers) / this, rows in neighbourhood order, on one B200:
 //   1,000,000 x 128, lists of 96 from near neighbours: 660 / 526
 //   60,007 x 768, lists of 192:                        155 / 121
 //   150,000 x 128, rounds 2 and 3:                  98, 97 / 76, 78
@@ -17,7 +17,7 @@
 // One warp per row and 20 rows per SM (vl_beam_solo) is better where a row's memo is small (32 KB or none, so that
 // 2,960 of them do not push each other out of L2) and its rows are short: searches of 30,000 x 96 (clusters)
 // 10.0 / 8.9 ms, 10,000 of 1,000,000 x 128 5.2 / 4.8, the first build round (no memo) of 150,000 x 128 253 / 227.  Rows
-// of 256 dimensions gain only where 20 rows per SM save a wave (2,500 searches: 1.54 / 1.08; first round of
+// of 256 dimensions gain only where 20 rows per SM save a wave (2,500 searches, memos of 64 KB: 1.54 / 1.08; first round of
 // 20,000: 44.8 / 46.9); 768 dimensions lose (3,000 searches: 3.3 / 4.9).
 #include "vl_beam_team.cuh"
 
@@ -52,10 +52,9 @@ int many_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, 
 // the choice described above
 bool vl_beam_solo(const vl_beam_params& p)
 {
-    if (p.dim > 256 || p.memo_entries > 4096) return false;
-    if (p.dim <= 128) return true;
+    if (p.dim <= 128) return p.memo_entries <= 4096;
     const int64_t sms = vl_sm_count();
-    return p.rows > sms * many_per_sm(2) && p.rows <= sms * many_per_sm(1);
+    return p.dim <= 256 && p.memo_entries <= 8192 && p.rows > sms * many_per_sm(2) && p.rows <= sms * many_per_sm(1);
 }
 
 template <int LPR, int JP, int JU, int METRIC, bool ALIGNED>
