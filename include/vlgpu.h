@@ -221,7 +221,8 @@ typedef struct vl_beam_params {
     unsigned long long* stats; /* optional [16] counters (added to): [1] gathered candidates, [2] search-queue merges,
                                   [3] visit-queue merges, [4] class-A candidates, [5] class-B rounds, [6] rows, [7] iterations */
     int32_t flags;             /* ignored (a row's phases overlap, so they have no cycle counters of their own) */
-    int32_t reserved;
+    int32_t wait_us;           /* longest wait of one row for the others of its batch (vl_beam_search_rows with
+                                  arrivals), in microseconds; <= 0 = 2 s */
     unsigned long long* row_ticket; /* optional device counter, zero at launch: warps then draw their next row from it
                                   (rows that take unequal time no longer wait for a fixed partner); NULL = fixed stride */
     int64_t group_row0;        /* row 0 of this launch sits at this position of the reference's host loop: its batch
@@ -242,7 +243,8 @@ int vl_beam_search(const vl_beam_params* params, void* stream);
  * all in flight at once, out_cols >= sq_len + pvc * graph_w and dump_last == 0; it then stores that
  * iteration in arrivals[n_checks] and every row holds head + that iteration's candidates as with
  * dump_last.  Otherwise arrivals[n_checks] stays 0 and the launch is vl_beam_search's.  A wait between
- * rows that runs out (2 s) sets VL_STATUS_TIMEOUT in *status. */
+ * rows that runs out (wait_us) sets VL_STATUS_TIMEOUT in *status: rows of the batch may then have ended at different
+ * iterations, so the caller clears its flag arrays and runs the batch again without arrivals, which waits for nothing. */
 int vl_beam_search_rows(const vl_beam_params* params, const int64_t* row_order, uint32_t* arrivals, void* stream);
 
 /* Sort keys for such an order when the rows searched are the indexed vectors [row_lo, row_hi)

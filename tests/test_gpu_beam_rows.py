@@ -76,6 +76,45 @@ def test_a_batch_that_stops_early_ends_together(built_lib):
     assert early > 0
 
 
+def flat_rows(seed, count, dim):
+    """Unit vectors of `dim` dimensions in a subspace of six: few neighbours are hard to find there."""
+    return torch.nn.functional.pad(rows_of(seed, count, 6, "cosine"), (0, dim - 6)).contiguous()
+
+
+def converging_index(degree, dim):
+    """An index whose searches settle long before their budget is spent: easy rows, a short search queue, a long visit queue."""
+    from vectorlink_gpu import ANN
+    return ANN(vectors=flat_rows(3, 4000, dim), beam_size=degree, visit_queue_factor=6, recall_search_queue_factor=1,
+               init="knn_tile", optimization_loops=1)
+
+
+def launches_of(ann, queries):
+    import vectorlink_gpu.ann as A
+    A.PROFILE = []
+    try:
+        ann.search(queries)
+        return len(A.PROFILE)
+    finally:
+        A.PROFILE = None
+
+
+@pytest.mark.parametrize("count", [200, 500, 1000])
+def test_a_wait_that_runs_out_is_answered_by_a_second_run(count, built_lib):
+    """Rows of a batch wait at most a microsecond for the others: some give up, and the batch is searched again without
+    waits.  The queues and the count are the operator path's, and no status bit stays behind."""
+    import vectorlink_gpu.ann as A
+    from vectorlink_gpu import _lib
+    ann = converging_index(16, 64)
+    queries = flat_rows(4, count, 64)
+    ann.configuration["wait_us"] = 1
+    launches = launches_of(ann, queries)
+    (fused, steps) = search_both_ways(ann, queries)
+    assert steps[2] <= A.loop_bounds(ann.configuration)[0]      # the batch does stop early
+    assert launches > 1
+    assert torch.equal(fused[0], steps[0]) and torch.equal(fused[1], steps[1]) and fused[2] == steps[2]
+    assert _lib.read_status(DEV) == 0
+
+
 @pytest.mark.parametrize("metric", ["cosine", "l2"])
 @pytest.mark.parametrize("dim,offset", [(1, 0), (3, 0), (50, 0), (127, 0), (255, 0), (511, 0), (1023, 0), (1027, 0), (64, 1), (96, 3)])
 def test_rows_without_whole_aligned_chunks_give_the_operator_path_results(dim, offset, metric, built_lib):

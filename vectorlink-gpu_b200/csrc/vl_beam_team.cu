@@ -10,7 +10,8 @@
 // agree on that check through one counter per check, so neither the iterations behind it nor a second
 // run up to it are spent.  A row that changed does not wait; one that did not waits until one that did or
 // all have reported.  The wait is bounded by wall time: when it runs out the row sets
-// VL_STATUS_TIMEOUT and goes on as if the batch had changed.
+// VL_STATUS_TIMEOUT and goes on as if the batch had changed.  Rows that saw the last report just before may then
+// have stopped, so the launch's results are of no use: the caller runs the batch again without `arrivals`.
 #include "vl_beam_team.cuh"
 
 namespace {

@@ -12,7 +12,7 @@ namespace {
 constexpr int kMaxTeam = 16;                                   // most warps per row
 // CTAs per SM that launches of many rows aim for: teams of one warp (96 registers) or two (64)
 constexpr int many_per_sm(int team) { return team == 1 ? 20 : 16; }
-constexpr unsigned long long kWaitLimitNs = 2000000000ull;     // 2 s per wait
+constexpr unsigned long long kWaitLimitNs = 2000000000ull;     // 2 s per wait, unless the caller asks for another limit
 
 struct TeamSmem {      // carve-up of the CTA's shared memory, in bytes
     int memo, query, cand, sq_a, sq_b, vq_a, vq_b, hash, todo, list_s, list_v, ctl, total;
@@ -476,7 +476,7 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
                             __threadfence();
                             atomicAdd(arrivals + chk, 1u);
                             if (!changed && waits) {
-                                const unsigned long long t0 = team_now_ns();
+                                const unsigned long long t0 = team_now_ns(), limit = p.wait_us > 0 ? p.wait_us * 1000ull : kWaitLimitNs;
                                 for (;;) {
                                     // all rows have reported, and none of them a change (a row's flag precedes its arrival)
                                     if (*(volatile unsigned int*)(arrivals + chk) >= (unsigned int)p.rows) {
@@ -485,7 +485,7 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
                                         break;
                                     }
                                     if (*(volatile unsigned int*)flag != 0) break;
-                                    if (team_now_ns() - t0 > kWaitLimitNs) {
+                                    if (team_now_ns() - t0 > limit) {
                                         atomicOr(p.status, VL_STATUS_TIMEOUT);
                                         atomicOr(flag, 1u);
                                         waits = false;

@@ -74,7 +74,7 @@ def loop_bounds(config: Dict) -> Tuple[int, int, int]:
 
 def _launch_beam(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_len, out_ids, out_dist, out_cols,
                  config, n_iters, dump_last, exclude, self_base, group_rows, flags, full, stats=None, group_row0=0,
-                 arrivals=None):
+                 arrivals=None, status=None):
     pvc = config["parallel_visit_count"]
     if stats is None:
         stats = STATS
@@ -114,11 +114,12 @@ def _launch_beam(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_len
     p.changed_flags = flags.data_ptr()
     p.n_checks = flags.size(1)
     p.group_full = full.data_ptr()
-    p.status = _lib.status_word(vectors.device).data_ptr()
+    p.status = (_lib.status_word(vectors.device) if status is None else status).data_ptr()
     p.memo = 0
     p.memo_slots = 0
     p.stats = stats.data_ptr() if stats is not None else 0
     p.flags = 0
+    p.wait_us = int(config.get("wait_us", 0))
     p.memo_entries = _memo_entries(p, config)
     smem, per_block, blocks = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
     check(lib().vl_beam_search_plan(ctypes.byref(p), ctypes.byref(smem), ctypes.byref(per_block), ctypes.byref(blocks)),
@@ -227,14 +228,15 @@ def _fused_batches(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_l
     nc = max(n_checks, 1)
     ng = max(total_groups, 1)
     # one buffer for both flag arrays: one all-reduce, one read-back
-    flag_buf = torch.zeros(ng * nc + ng + nc + 1, dtype=torch.int32, device=dev)
+    flag_buf = torch.zeros(ng * nc + ng + nc + 2, dtype=torch.int32, device=dev)
     flags = flag_buf[: ng * nc].view(ng, nc)
     full = flag_buf[ng * nc: ng * nc + ng]
     # one batch whose rows are all in flight at once may end together at the check at which the reference
-    # leaves (the kernel then stores that iteration in the last word) instead of being run again up to it
+    # leaves (the kernel then stores that iteration in the last word of `arrivals`) instead of being run again up
+    # to it.  Such a launch waits between rows, and a wait can run out, so it gets a status word of its own
     together = {}
     if rows and reduce_group is None and ng == 1 and out_cols == sq_cap and out_ids.is_cuda and out_ids.is_contiguous():
-        together = {"arrivals": flag_buf[ng * nc + ng:]}
+        together = {"arrivals": flag_buf[ng * nc + ng: -1], "status": flag_buf[-1:]}
     if rows == 0 and reduce_group is None:
         return []
     # a caller that wants to know how useful the distance memo is on this graph (generate_ann's
@@ -242,10 +244,13 @@ def _fused_batches(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_l
     counters = None
     if config.get("measure_gathered") and config.get("memo", True):
         counters = torch.zeros(24, dtype=torch.int64, device=dev)
-    if rows:
+
+    def launch(**more):
         _launch_beam(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_len, out_ids, out_dist, out_cols,
-                     config, n_max, False, exclude, self_base, group_rows, flags, full, counters, group_row0,
-                     **together)
+                     config, n_max, False, exclude, self_base, group_rows, flags, full, counters, group_row0, **more)
+
+    if rows:
+        launch(**together)
     if reduce_group is not None:
         import torch.distributed as dist
         with nvtx_range("vl.flags_allreduce"):
@@ -253,9 +258,17 @@ def _fused_batches(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_l
     if rows == 0:
         return []
     host = flag_buf.cpu()
+    if int(host[-1]):
+        # a wait ran out, and rows may have ended at different iterations (or an id was bad, which the device's
+        # status word has to say): the same batch without waits
+        flag_buf.zero_()
+        if counters is not None:
+            counters.zero_()
+        launch()
+        host = flag_buf.cpu()
     flags_h = host[: ng * nc].view(ng, nc).tolist()
     full_h = host[ng * nc: ng * nc + ng].tolist()
-    ended = int(host[-1])
+    ended = int(host[-2])
     if counters is not None:
         if STATS is not None:
             shared = min(STATS.numel(), counters.numel())
