@@ -1,0 +1,63 @@
+"""Calls of several host threads, each on a stream of its own: what one of them keeps or shares must not reach the others."""
+import threading
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def unit_rows(seed, count, dim):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(seed)
+    return torch.nn.functional.normalize(torch.randn((count, dim), generator=g, device=DEV), dim=1)
+
+
+def serial_and_threaded(calls, passes):
+    """What every call gives by itself, and what it gives `passes` times in a thread and stream of its own while the
+    others run: each stream is busy for some milliseconds first, so that the launches of a pass start together."""
+    serial = []
+    for call in calls:
+        queue = call()
+        serial.append((queue.indices.clone(), queue.distances.clone()))
+    torch.cuda.synchronize()
+    got = [[] for _ in calls]
+    gate = threading.Barrier(len(calls))
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(passes):
+                gate.wait(60)
+                try:
+                    torch.cuda._sleep(20_000_000)
+                    queue = calls[i]()
+                    got[i].append((queue.indices.clone(), queue.distances.clone()))
+                    torch.cuda.current_stream().synchronize()
+                except Exception as e:      # the other threads still meet this one at the gate
+                    got[i].append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(calls))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    return serial, got
+
+
+def assert_threads_change_nothing(calls, passes=10):
+    (serial, got) = serial_and_threaded(calls, passes)
+    for (want, passes_of_one) in zip(serial, got):
+        for one in passes_of_one:
+            assert not isinstance(one, Exception), one
+            assert torch.equal(one[0], want[0]) and torch.equal(one[1], want[1])
+
+
+@pytest.mark.parametrize("count", [1300, 2000])     # memos in global memory, and room on the chip for both launches
+def test_searches_of_two_streams_share_no_memo(count, built_lib):
+    from vectorlink_gpu import ANN
+    index = ANN(vectors=unit_rows(1, 3000, 128), beam_size=16, visit_queue_factor=2, recall_search_queue_factor=2,
+                init="knn_tile", optimization_loops=1)
+    (a, b) = (unit_rows(2, count, 128), unit_rows(3, count, 128))
+    assert_threads_change_nothing([lambda: index.search(a), lambda: index.search(b)])

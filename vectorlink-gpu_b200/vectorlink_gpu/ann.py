@@ -129,9 +129,10 @@ def _launch_beam(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_len
     ticket = torch.zeros(1, dtype=torch.int64, device=vectors.device) if scratch and config.get("row_ticket", True) else None
     p.row_ticket = ticket.data_ptr() if ticket is not None else 0
     if scratch and p.memo_entries:
-        # id -> distance memo of each row in flight (scratch; the kernel clears a row's slice)
+        # id -> distance memo of each row in flight (the kernel clears a row's slice).  Scratch of this launch alone:
+        # an entry does not say whose query its distance is of, so launches of other streams must not meet it
         slots = max(1, per_block.value * blocks.value)
-        memo = _memo_buffer(vectors.device, slots * p.memo_entries)
+        memo = torch.empty(slots * p.memo_entries, dtype=torch.int64, device=vectors.device)
         p.memo = memo.data_ptr()
         p.memo_slots = slots
     order = _row_order(graph, self_base, queries.size(0), config) if p.memo else None
@@ -181,19 +182,6 @@ def _memo_entries(p: BeamParams, config: Dict) -> int:
         while entries < need and entries < 16384:
             entries *= 2
     return entries
-
-
-_memo_cache = {}
-
-
-def _memo_buffer(device, words: int) -> Tensor:
-    """A reusable int64 scratch tensor of at least `words` entries on `device`."""
-    key = _lib._device_key(device)
-    buf = _memo_cache.get(key)
-    if buf is None or buf.numel() < words:
-        buf = torch.empty(words, dtype=torch.int64, device=key)
-        _memo_cache[key] = buf
-    return buf
 
 
 def _natural_end(flag_row: List[int], config: Dict) -> int:
