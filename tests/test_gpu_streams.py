@@ -61,3 +61,43 @@ def test_searches_of_two_streams_share_no_memo(count, built_lib):
                 init="knn_tile", optimization_loops=1)
     (a, b) = (unit_rows(2, count, 128), unit_rows(3, count, 128))
     assert_threads_change_nothing([lambda: index.search(a), lambda: index.search(b)])
+
+
+@pytest.mark.parametrize("metric", ["cosine", "l2"])
+def test_entry_points_of_two_streams_are_their_own(metric, built_lib):
+    from vectorlink_gpu import ANN
+    index = ANN(vectors=unit_rows(1, 20_000, 128), beam_size=16, visit_queue_factor=2, recall_search_queue_factor=2,
+                metric=metric, init="knn_tile", optimization_loops=1, search_entry_sample=16_384)
+    (a, b) = (unit_rows(2, 500, 128), unit_rows(3, 700, 128))
+    assert_threads_change_nothing([lambda: index.search(a), lambda: index.search(b)], passes=30)
+
+
+def test_the_entry_sample_is_complete_before_another_stream_meets_it(built_lib):
+    """The first search of an index makes the sample on a stream that is busy; a search on another stream, started right
+    after the sample is there, must not read it half made.  (Both streams have met another index first: their memory is
+    allocated, which the device would be waited for, and holds other rows.)"""
+    from vectorlink_gpu import ANN
+    def index_of(seed):
+        vectors = unit_rows(seed, 20_000, 128)
+        return ANN(vectors=vectors, beams=torch.zeros((20_000, 16), dtype=torch.int32, device=DEV), beam_size=16,
+                   search_entry_sample=16_384)
+
+    queries = unit_rows(2, 500, 128)
+    (other, index) = (index_of(4), index_of(1))
+    want = index._entry_seeds(queries)
+    index._entry = None
+    (first, second) = (torch.cuda.Stream(), torch.cuda.Stream())
+    for stream in (first, second):
+        with torch.cuda.stream(stream):
+            other._entry = None
+            other._entry_seeds(queries)
+            stream.synchronize()
+    other._entry = None
+    torch.cuda.synchronize()
+    with torch.cuda.stream(first):
+        torch.cuda._sleep(200_000_000)
+        index._entry_seeds(queries)
+    with torch.cuda.stream(second):
+        got = index._entry_seeds(queries)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)

@@ -65,7 +65,7 @@ def proposals(rows_bf16: Tensor, norms: Optional[Tensor], rows: Tuple[int, int],
     """int32 [rows, segments * 64]: per row and per part of the candidate range (`segments` equal
     parts) four lists of 16 ids: list k holds the best-scoring candidates among the k-th quarters
     (64 candidates) of the part's 256-candidate tiles (approximate scores; the row itself excluded),
-    MAXINT-padded."""
+    MAXINT-padded.  `norms`: of every row up to candidates[1]; only candidates' are read."""
     _lib.require_cuda(rows_bf16, norms)
     assert rows_bf16.dtype == torch.bfloat16 and rows_bf16.is_contiguous()
     (n, dim_pad) = rows_bf16.size()
