@@ -101,3 +101,39 @@ def test_the_entry_sample_is_complete_before_another_stream_meets_it(built_lib):
         got = index._entry_seeds(queries)
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+def test_a_plan_of_another_thread_does_not_refuse_a_launch(built_lib):
+    """One kernel, rows of two sizes: a thread that plans launches of small rows must not take the shared memory from under
+    the launches of another thread, whose rows need more than the 48 KB that every kernel may have."""
+    import ctypes
+    from vectorlink_gpu import ANN
+    from vectorlink_gpu._lib import BeamParams, lib
+    vectors = unit_rows(1, 20_000, 128)
+    index = ANN(vectors=vectors, beam_size=32, visit_queue_factor=25, recall_search_queue_factor=4, init="knn_tile",
+                optimization_loops=0)
+    index.configuration["memo"] = False
+    queries = unit_rows(2, 1200, 128)
+    want = index.search(queries).indices.clone()
+    some = vectors.data_ptr()           # a plan reads no memory
+    small = BeamParams(vectors=some, n=20_000, dim=128, graph=some, graph_w=16, pvc=4, queries=some, rows=1200, seed_ids=some,
+                       seed_dist=some, seed_ld=32, seed_cols=32, sq_len=32, vq_len=32, seen_cap=160, out_ids=some, out_dist=some,
+                       out_ld=32, out_cols=32, n_iters=45, readahead=5, self_base=-1, changed_flags=some, group_full=some, status=some)
+    (size, per_block, blocks) = (ctypes.c_int(), ctypes.c_int(), ctypes.c_int())
+    stop = threading.Event()
+    refused = []
+
+    def plan():
+        while not stop.is_set():
+            if lib().vl_beam_search_plan(ctypes.byref(small), ctypes.byref(size), ctypes.byref(per_block), ctypes.byref(blocks)):
+                refused.append(lib().vl_last_error())
+
+    planner = threading.Thread(target=plan)
+    planner.start()
+    try:
+        for _ in range(60):
+            assert torch.equal(index.search(queries).indices, want)
+    finally:
+        stop.set()
+        planner.join()
+    assert not refused and blocks.value > 0

@@ -31,6 +31,14 @@ int vl_sm_count()
     return cached[dev];
 }
 
+int vl_smem_limit()
+{
+    int dev = 0, bytes = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
+    return bytes;
+}
+
 extern "C" const char* vl_last_error(void) { return g_error; }
 
 extern "C" int vl_abi_version(void) { return 4; }

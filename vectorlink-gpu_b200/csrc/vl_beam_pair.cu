@@ -28,12 +28,10 @@ int many_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, 
 {
     auto kernel = beam_team_kernel<LPR, JP, JU, METRIC, ALIGNED, TEAM>;
     const TeamSmem lay = team_layout(p.pvc * p.graph_w, p.sq_len, p.vq_len, p.seen_cap, LPR * JP * 16, p.memo ? p.memo_entries : 0, false);
-    int dev = 0, max_smem = 0, per_sm = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    VL_CHECK_ARG(e == cudaSuccess, "vl_beam_search: %s", cudaGetErrorString(e));
-    VL_CHECK_ARG(lay.total <= max_smem, "vl_beam_search: one row needs %d bytes of shared memory, the device offers %d", lay.total, max_smem);
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lay.total);
+    int per_sm = 0;
+    VL_CHECK_ARG(lay.total <= vl_smem_limit(), "vl_beam_search: one row needs %d bytes of shared memory, the device offers %d", lay.total,
+                 vl_smem_limit());
+    cudaError_t e = vl_allow_smem(kernel);
     VL_CHECK_ARG(e == cudaSuccess, "vl_beam_search: %s", cudaGetErrorString(e));
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * TEAM, lay.total);
     VL_CHECK_ARG(e == cudaSuccess && per_sm > 0, "vl_beam_search: occupancy query failed");

@@ -35,11 +35,8 @@ bool team_plan(const vl_beam_params& p, TeamPlan& plan)
     else if (per_sm <= 8) plan.warps = 2;
     else return false;
     plan.per_sm = kMaxTeam / plan.warps;
-    int dev = 0, max_smem = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return false;
     const VlShape shape = vl_pick_shape(p.dim);
-    const int budget = max_smem / plan.per_sm - 1024;
+    const int budget = vl_smem_limit() / plan.per_sm - 1024;
     // the memo holds the ids a row gathers: about a quarter of the neighbours it looks at
     int entries = 1024;
     while (entries < 16384 && entries < (int64_t)p.seen_cap * p.graph_w / 4) entries <<= 1;
@@ -57,7 +54,7 @@ int team_launch(const vl_beam_params& p, const TeamPlan& plan, unsigned int* arr
 {
     auto kernel = beam_team_kernel<LPR, JP, JU, METRIC, ALIGNED, kMaxTeam>;
     TeamSmem lay = plan.lay;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lay.total);
+    cudaError_t e = vl_allow_smem(kernel);
     VL_CHECK_ARG(e == cudaSuccess, "vl_beam_search: %s", cudaGetErrorString(e));
     const int64_t slots = (int64_t)vl_sm_count() * plan.per_sm;
     const unsigned grid = (unsigned)(p.rows < slots ? p.rows : slots);

@@ -377,6 +377,15 @@ static inline VlShape vl_pick_shape(int dim)
 // host-side error plumbing shared by the extern "C" entry points
 void vl_set_error(const char* fmt, ...);
 int vl_sm_count();   // SMs of the current device
+int vl_smem_limit(); // bytes of shared memory that a CTA may ask for on the current device (0 if it cannot be asked)
+// Lets a kernel take as much dynamic shared memory as a CTA may ask for.  The limit belongs to the kernel and not
+// to one launch, so it always gets the same value: a thread that set it to what its own launch needs would
+// have the launch of another thread, with a larger row, refused.
+template <typename Kernel>
+inline cudaError_t vl_allow_smem(Kernel kernel)
+{
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, vl_smem_limit());
+}
 #define VL_CHECK_ARG(cond, ...)          \
     do {                                 \
         if (!(cond)) {                   \

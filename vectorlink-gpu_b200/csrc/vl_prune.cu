@@ -134,7 +134,7 @@ extern "C" int vl_prune_rows(const int32_t* beams, const float* dist, int64_t n,
     size_t per_warp = (size_t)p + 2 * (size_t)((w + 1) / 2) * 2;
     size_t smem = per_warp * sizeof(vl_key_t) * kPruneWarps;
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(prune_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = vl_allow_smem(prune_kernel);
         VL_CHECK_ARG(e == cudaSuccess, "vl_prune: %s", cudaGetErrorString(e));
     }
     int64_t blocks = (row_hi - row_lo + kPruneWarps - 1) / kPruneWarps;
