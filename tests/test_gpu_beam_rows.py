@@ -53,6 +53,60 @@ def test_one_or_two_warps_per_row_give_the_same_queues(count, memo, built_lib):
     assert torch.equal(fused[0], steps[0]) and torch.equal(fused[1], steps[1]) and fused[2] == steps[2]
 
 
+@pytest.mark.parametrize("dim,memo", [(64, {}), (64, {"memo": False}), (512, {})])      # two, one and two warps per row
+@pytest.mark.parametrize("degree,pvc,exclude_w", [(64, 4, 0), (64, 4, 3), (32, 16, 3), (33, 4, 0)])
+def test_wide_lists_with_and_without_exclusions(degree, pvc, exclude_w, dim, memo, built_lib):
+    """Iterations of 132 to 512 candidates, with exclusion lists and without, and with 16 ids popped at once (the visit
+    queue is then offered every candidate), at a row count of one or two warps per row."""
+    import vectorlink_gpu.ann as A
+    count = 1300
+    ann = A.ANN(vectors=rows_of(1, 3001, dim, "cosine"), beam_size=degree, visit_queue_factor=2, recall_search_queue_factor=2,
+                parallel_visit_count=pvc, init="knn_tile", optimization_loops=1)
+    queries = rows_of(2, count, dim, "cosine")
+    exclude = None
+    if exclude_w:
+        exclude = ann.search(queries).indices[:, :exclude_w].contiguous()      # the nearest ones may not be found
+        exclude[::2, -1] = 2147483647
+    got = []
+    for more in (memo, {"stepwise": True}):
+        queue = A.initial_search_queue(ann.vectors, queries, ann.configuration)
+        A.closest_vectors(queries, queue, ann.vectors, ann.beams, dict(ann.configuration, **more), exclude)
+        got.append((queue.indices, queue.distances, A.closest_vectors.last_count))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and got[0][2] == got[1][2]
+
+
+@pytest.mark.parametrize("degree,width,dim,visits,exclude", [(128, 384, 32, 3, 5), (128, 384, 300, 3, 5), (520, 520, 32, 1, 1)])
+def test_rows_of_many_candidates_per_iteration_are_fused(degree, width, dim, visits, exclude, built_lib):
+    """12,288 and 16,640 candidates per iteration, which the operator path refuses, against the oracle.  With lists of
+    entrants the last needs more shared memory than a CTA can have.  (The one check comes after the budget: a batch that
+    ends early is sorted whole, and rows of this capacity are refused there.)"""
+    import oracle
+    import vectorlink_gpu.ann as A
+    config = oracle.make_config(beam_size=degree, parallel_visit_count=32, visit_queue_factor=visits, exclude_factor=exclude)
+    config["speculative_readahead"] = A.loop_bounds(config)[0] + 1
+    rng = np.random.default_rng(degree)
+    vectors = rng.standard_normal((20_000, dim), dtype=np.float32)
+    vectors /= np.linalg.norm(vectors, axis=1, keepdims=True)
+    graph = rng.integers(0, 20_000, (20_000, width)).astype(np.int32)
+    queries = vectors[:3].copy()
+    m = 32 * width
+    queue = oracle.Queue(3, width, width + m)
+    queue.insert(graph[:3], oracle.calculate_distances(vectors, graph)[:3])
+    mine = A.Queue(3, width, width + m)
+    mine.indices.copy_(torch.from_numpy(queue.indices))
+    mine.distances.copy_(torch.from_numpy(queue.distances))
+    A.PROFILE = []
+    try:
+        A.closest_vectors(torch.from_numpy(queries).to(DEV), mine, torch.from_numpy(vectors).to(DEV), torch.from_numpy(graph).to(DEV), config)
+        assert len(A.PROFILE) > 0
+    finally:
+        A.PROFILE = None
+    count = oracle.closest_vectors(queries, queue, vectors, graph, config)
+    assert A.closest_vectors.last_count == count
+    assert np.array_equal(mine.indices[:, :width].cpu().numpy(), queue.indices[:, :width])
+    assert np.array_equal(mine.distances[:, :width].cpu().numpy(), queue.distances[:, :width])
+
+
 def test_a_batch_that_stops_early_ends_together(built_lib):
     """Few rows stop at the reference's check: one launch, no second run up to it."""
     import vectorlink_gpu.ann as A

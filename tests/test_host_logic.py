@@ -121,3 +121,14 @@ def test_tile_pass_wrappers_refuse_cpu_tensors(built_lib):
     import pytest as _pytest
     with _pytest.raises(_lib.VlError):
         knn_tile.prepare(torch.zeros(4, 64), want_norms=True)
+
+
+def test_wide_lists_stay_fused():
+    """Graph widths and visit counts up to 200 KB of candidates, queues and visited ids per row go to the fused search."""
+    from vectorlink_gpu.ann import _fused_queue_ok
+    for (degree, pvc, factor, width) in ((128, 32, 3, 384), (64, 32, 2, 192), (256, 16, 2, 768), (24, 4, 3, 72)):
+        config = {"parallel_visit_count": pvc, "visit_queue_factor": factor, "beam_size": degree, "exclude_factor": 5,
+                  "speculative_readahead": 5}
+        (m, visits) = (pvc * width, factor * degree)
+        if 10 * m + 16 * width + 16 * visits + 24 * 5 * visits + 4 * 1536 + 512 <= 200 * 1024:
+            assert _fused_queue_ok(width, width, width + m, config), (degree, pvc)

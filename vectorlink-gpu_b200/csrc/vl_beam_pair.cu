@@ -23,11 +23,17 @@
 
 namespace {
 
+template <int TEAM, int LPR, int JP>
+TeamSmem many_layout(const vl_beam_params& p)
+{
+    return team_layout(p.pvc * p.graph_w, p.sq_len, p.vq_len, p.seen_cap, LPR * JP * 16, p.memo ? p.memo_entries : 0, false, TEAM > 1);
+}
+
 template <int TEAM, int LPR, int JP, int JU, int METRIC, bool ALIGNED>
 int many_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)
 {
     auto kernel = beam_team_kernel<LPR, JP, JU, METRIC, ALIGNED, TEAM>;
-    const TeamSmem lay = team_layout(p.pvc * p.graph_w, p.sq_len, p.vq_len, p.seen_cap, LPR * JP * 16, p.memo ? p.memo_entries : 0, false);
+    const TeamSmem lay = many_layout<TEAM, LPR, JP>(p);
     int per_sm = 0;
     VL_CHECK_ARG(lay.total <= vl_smem_limit(), "vl_beam_search: one row needs %d bytes of shared memory, the device offers %d", lay.total,
                  vl_smem_limit());
@@ -58,9 +64,9 @@ bool vl_beam_solo(const vl_beam_params& p)
 template <int LPR, int JP, int JU, int METRIC, bool ALIGNED>
 int pair_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)
 {
-    if constexpr (LPR * JP <= 64) {     // 256 dimensions
-        if (vl_beam_solo(p)) return many_launch<1, LPR, JP, JU, METRIC, ALIGNED>(p, row_order, launch, blocks, smem, stream);
-    }
+    // a single warp needs 10 instead of 14 bytes of shared memory per candidate: rows of more than about 15,000 take it
+    if (vl_beam_solo(p) || many_layout<2, LPR, JP>(p).total > vl_smem_limit())
+        return many_launch<1, LPR, JP, JU, METRIC, ALIGNED>(p, row_order, launch, blocks, smem, stream);
     return many_launch<2, LPR, JP, JU, METRIC, ALIGNED>(p, row_order, launch, blocks, smem, stream);
 }
 

@@ -43,7 +43,7 @@ bool team_plan(const vl_beam_params& p, TeamPlan& plan)
     // (with less than a quarter of that, gathers repeated cost more than the warps save: 1,000 rows of 768
     // dimensions with 1,024 of 16,384 entries 7.7 ms, vl_beam_pair.cu 3.6 ms)
     for (const int least = entries / 4 > 1024 ? entries / 4 : 1024; entries >= least; entries >>= 1) {
-        plan.lay = team_layout((int)m, p.sq_len, p.vq_len, p.seen_cap, shape.lpr * shape.jp * 16, entries, true);
+        plan.lay = team_layout((int)m, p.sq_len, p.vq_len, p.seen_cap, shape.lpr * shape.jp * 16, entries, true, true);
         if (plan.lay.total <= budget) return true;
     }
     return false;

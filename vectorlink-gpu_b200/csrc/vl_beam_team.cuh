@@ -19,8 +19,10 @@ struct TeamSmem {      // carve-up of the CTA's shared memory, in bytes
     int hash_slots, hash_shift, memo_buckets, memo_shift;
 };
 
-// memo_entries: entries of the row's distance memo, 0 = none; on_chip: they are in shared memory
-__host__ inline TeamSmem team_layout(int m, int sq_len, int vq_len, int seen_cap, int query_bytes, int memo_entries, bool on_chip)
+// memo_entries: entries of the row's distance memo, 0 = none; on_chip: they are in shared memory; lists: space for the
+// lists of entrants (a single warp makes them one after the other in the place of `todo`)
+__host__ inline TeamSmem team_layout(int m, int sq_len, int vq_len, int seen_cap, int query_bytes, int memo_entries, bool on_chip,
+                                     bool lists)
 {
     TeamSmem s;
     int off = 0;
@@ -41,8 +43,8 @@ __host__ inline TeamSmem team_layout(int m, int sq_len, int vq_len, int seen_cap
     s.hash = off; off += 4 * slots;
     s.ctl = off; off += 4 * 16;
     s.todo = off; off += 2 * m;
-    s.list_s = off; off += 2 * m;
-    s.list_v = off; off += 2 * m;
+    s.list_s = lists ? off : s.todo; off += lists ? 2 * m : 0;
+    s.list_v = lists ? off : s.todo; off += lists ? 2 * m : 0;
     s.total = (off + 15) & ~15;
     return s;
 }
@@ -417,6 +419,7 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
             const vl_key_t cut = sq[sq_len - 1];
             const bool usual = seen_live && n_old > 0 && vq_len - n_old <= 8;
             const vl_key_t t0key = n_old > 0 ? vq[n_old - 1 + pvc] : kSent;
+            int n_entrants = 0;                       // of the search queue, in list_s (one warp per row)
 #pragma unroll 1
             for (int t0 = warp * 32; t0 < n_todo; t0 += threads) {
                 const int t = t0 + lane;
@@ -427,9 +430,15 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
                     const int32_t id = vl_key_id(key);
                     if (id == self_id || (excl && team_excluded(excl, p.exclude_w, id))) want = false;
                 }
-                team_append(list_s, ctl_count + kListS, want, c, lane);
+                if constexpr (TEAM == 1) {            // list_s is todo: never ahead of the reads, which this ballot waits for
+                    const unsigned mask = __ballot_sync(0xffffffffu, want);
+                    if (want) list_s[n_entrants + __popc(mask & ((1u << lane) - 1u))] = (unsigned short)c;
+                    n_entrants += __popc(mask);
+                } else {
+                    team_append(list_s, ctl_count + kListS, want, c, lane);
+                }
             }
-            if (usual) {
+            if (TEAM > 1 && usual) {
 #pragma unroll 1
                 for (int c0 = warp * 32; c0 < m_total; c0 += threads) {
                     const int c = c0 + lane;
@@ -441,7 +450,7 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
             if (warp == 0) {
                 // ---- search_queue.insert(..., exclude) (ann.py:75-80) ----
                 bool changed = false;
-                const int n_in = ctl[kListS];
+                const int n_in = TEAM == 1 ? n_entrants : ctl[kListS];
                 int held = ctl[kHeld];
                 if (n_in) {
                     vl_key_t* sq_n = reinterpret_cast<vl_key_t*>(smem + (lay.sq_a + lay.sq_b - ctl[kSqBuf]));
@@ -500,6 +509,12 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
             }
             if (warp == (TEAM == 1 ? 0 : 1)) {
                 // ---- the popped heads leave, visit_queue.insert(..., exclude=seen) ----
+                if (TEAM == 1 && usual) {
+#pragma unroll 1
+                    for (int c0 = 0; c0 < m_total; c0 += 32)
+                        team_append(list_v, ctl_count + kListV, c0 + lane < m_total && candk[c0 + lane] < t0key, c0 + lane, lane);
+                    __syncwarp();
+                }
                 vl_key_t* vq_n = reinterpret_cast<vl_key_t*>(smem + (lay.vq_a + lay.vq_b - ctl[kVqBuf]));
                 const int n_a = usual ? ctl[kListV] : (seen_live ? m_total : 0);   // an (almost) empty queue is offered every candidate
                 st_a += usual ? n_a : 0;

@@ -46,7 +46,8 @@ def _fused_queue_ok(beam_w: int, sq_len: int, sq_cap: int, config: Dict) -> bool
     vq_len = config["visit_queue_factor"] * config["beam_size"]
     m = pvc * beam_w
     e = config["exclude_factor"] * vq_len
-    smem = 14 * m + 16 * sq_len + 16 * vq_len + 4 * 6 * max(e, 16) + 4 * 1024 + 512
+    # (beside these a row keeps its query, 4 KB at most: the device offers 227 KB)
+    smem = 10 * m + 16 * sq_len + 16 * vq_len + 4 * 6 * max(e, 16) + 512
     return (1 <= pvc <= 32 and pvc <= vq_len and sq_cap == sq_len + m and sq_len <= 4096 and m <= 65535
             and smem <= FUSED_MAX_SMEM_PER_ROW and config["speculative_readahead"] >= 1)
 
