@@ -53,6 +53,29 @@ def test_one_or_two_warps_per_row_give_the_same_queues(count, memo, built_lib):
     assert torch.equal(fused[0], steps[0]) and torch.equal(fused[1], steps[1]) and fused[2] == steps[2]
 
 
+@pytest.mark.parametrize("width,memo_entries", [(16, 0), (48, 0), (52, 8192), (64, 0), (128, 0)])
+def test_one_warp_per_row_is_chosen_by_the_rows_that_fit(width, memo_entries, built_lib):
+    """256 dimensions, where shared memory allows 20 or fewer rows per SM: the plan never leaves rows to a second wave because of
+    one warp per row, and keeps all rows in flight where two warps per row would not."""
+    import ctypes
+    from vectorlink_gpu._lib import BeamParams, check, lib
+    some = torch.zeros(4, device=DEV).data_ptr()           # a plan reads no memory
+
+    def planned(rows):
+        p = BeamParams(vectors=some, n=20_000, dim=256, graph=some, graph_w=width, pvc=4, queries=some, rows=rows, seed_ids=some,
+                       seed_dist=some, seed_ld=2 * width, seed_cols=2 * width, sq_len=2 * width, vq_len=2 * width, seen_cap=10 * width,
+                       out_ids=some, out_dist=some, out_ld=2 * width, out_cols=2 * width, n_iters=10, readahead=5, self_base=-1,
+                       changed_flags=some, group_full=some, status=some, memo_entries=memo_entries)
+        (size, per_block, blocks) = (ctypes.c_int(), ctypes.c_int(), ctypes.c_int())
+        check(lib().vl_beam_search_plan(ctypes.byref(p), ctypes.byref(size), ctypes.byref(per_block), ctypes.byref(blocks)), "plan")
+        return blocks.value
+
+    two_warps = planned(100_000)                           # rows in flight with two warps per row
+    blocks = [planned(rows) for rows in range(1200, 3200, 20)]
+    for rows, b in zip(range(1200, 3200, 20), blocks):
+        assert b == (rows if b > two_warps else min(rows, two_warps)), rows
+
+
 @pytest.mark.parametrize("dim,memo", [(64, {}), (64, {"memo": False}), (512, {})])      # two, one and two warps per row
 @pytest.mark.parametrize("degree,pvc,exclude_w", [(64, 4, 0), (64, 4, 3), (32, 16, 3), (33, 4, 0)])
 def test_wide_lists_with_and_without_exclusions(degree, pvc, exclude_w, dim, memo, built_lib):

@@ -14,11 +14,17 @@
 // registers (two gather steps in flight): 541, 119, 81; one warp per row with the same queue step at 16 rows per
 // SM: 528, 137, 75, at 24 rows per SM: 740, 144, 108.
 //
-// One warp per row and 20 rows per SM (vl_beam_solo) is better where a row's memo is small (32 KB or none, so that
-// 2,960 of them do not push each other out of L2) and its rows are short: searches of 30,000 x 96 (clusters)
-// 10.0 / 8.9 ms, 10,000 of 1,000,000 x 128 5.2 / 4.8, the first build round (no memo) of 150,000 x 128 253 / 227.  Rows
-// of 256 dimensions gain only where 20 rows per SM save a wave (2,500 searches, memos of 64 KB: 1.54 / 1.08; first round of
-// 20,000: 44.8 / 46.9); 768 dimensions lose (3,000 searches: 3.3 / 4.9).
+// One warp per row and 20 rows per SM is better where a row's memo is small (32 KB or none, so that 2,960 of them do not
+// push each other out of L2) and its rows are short: searches of 30,000 x 96 (clusters) 10.0 / 8.9 ms, 10,000 of
+// 1,000,000 x 128 5.2 / 4.8, the first build round (no memo) of 150,000 x 128 253 / 227.  That also holds where shared memory
+// and not registers bounds the rows in flight (wide lists; first rounds without memo of 10,000 to 60,000 rows, two warps /
+// one warp): 128 dimensions at degree 40, 48, 64, 80, 96, 128, 192: 160 / 137, 233 / 205, 441 / 401, 408 / 383, 652 / 602,
+// 910 / 912, 1,758 / 1,547; 64 dimensions at 64, 80, 96: 271 / 250, 258 / 238, 410 / 374; 32 and 100 dimensions at 64: 248 / 235,
+// 527 / 415.  Only rows of 96 dimensions go the other way from degree 56 on (254 / 261; 64, 80, 96: 333 / 350, 293 / 331, 456 / 522).
+// Rows of 256 dimensions gain only where one warp per row keeps a launch in flight that two warps do not: with memos of 64 KB
+// 2,368 searches 2.40 / 2.68, 2,500 3.47 / 2.79, 2,960 3.68 / 3.09, 3,100 3.81 / 5.05.  A second wave saved gains nothing (4,800,
+// 5,300, 5,900 searches 5.94 / 5.85, 6.05 / 6.21, 6.44 / 6.61; CTAs draw their next row as they finish, so waves blur); first round of
+// 20,000: 44.8 / 46.9; 768 dimensions lose (3,000 searches: 3.3 / 4.9).
 #include "vl_beam_team.cuh"
 
 namespace {
@@ -29,44 +35,49 @@ TeamSmem many_layout(const vl_beam_params& p)
     return team_layout(p.pvc * p.graph_w, p.sq_len, p.vq_len, p.seen_cap, LPR * JP * 16, p.memo ? p.memo_entries : 0, false, TEAM > 1);
 }
 
+// CTAs = rows of this launch that the device keeps in flight at once; 0 if a row does not fit, -1 on an error
 template <int TEAM, int LPR, int JP, int JU, int METRIC, bool ALIGNED>
-int many_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)
+int64_t rows_in_flight(const vl_beam_params& p)
 {
     auto kernel = beam_team_kernel<LPR, JP, JU, METRIC, ALIGNED, TEAM>;
     const TeamSmem lay = many_layout<TEAM, LPR, JP>(p);
+    if (lay.total > vl_smem_limit()) return 0;
     int per_sm = 0;
+    if (vl_allow_smem(kernel) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * TEAM, lay.total) != cudaSuccess) return -1;
+    return (int64_t)vl_sm_count() * per_sm;
+}
+
+template <int TEAM, int LPR, int JP, int JU, int METRIC, bool ALIGNED>
+int many_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)
+{
+    const TeamSmem lay = many_layout<TEAM, LPR, JP>(p);
     VL_CHECK_ARG(lay.total <= vl_smem_limit(), "vl_beam_search: one row needs %d bytes of shared memory, the device offers %d", lay.total,
                  vl_smem_limit());
-    cudaError_t e = vl_allow_smem(kernel);
-    VL_CHECK_ARG(e == cudaSuccess, "vl_beam_search: %s", cudaGetErrorString(e));
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * TEAM, lay.total);
-    VL_CHECK_ARG(e == cudaSuccess && per_sm > 0, "vl_beam_search: occupancy query failed");
-    const int64_t resident = (int64_t)vl_sm_count() * per_sm;   // one resident wave; further rows are drawn as CTAs finish
+    const int64_t resident = rows_in_flight<TEAM, LPR, JP, JU, METRIC, ALIGNED>(p);   // one wave; further rows are drawn as CTAs finish
+    VL_CHECK_ARG(resident > 0, "vl_beam_search: occupancy query failed");
     const int grid = (int)(p.rows < resident ? p.rows : resident);
     *blocks = grid;
     *smem = lay.total;
     if (!launch) return 0;
     VL_CHECK_ARG(!p.memo || p.memo_slots >= grid, "vl_beam_search: memo has %lld slots, the launch keeps %d rows in flight",
                  (long long)p.memo_slots, grid);
-    kernel<<<grid, 32 * TEAM, lay.total, stream>>>(p, lay, row_order, nullptr);
+    beam_team_kernel<LPR, JP, JU, METRIC, ALIGNED, TEAM><<<grid, 32 * TEAM, lay.total, stream>>>(p, lay, row_order, nullptr);
     VL_CHECK_LAUNCH("beam_team_kernel");
     return 0;
-}
-
-// the choice described above
-bool vl_beam_solo(const vl_beam_params& p)
-{
-    if (p.dim <= 128) return p.memo_entries <= 4096;
-    const int64_t sms = vl_sm_count();
-    return p.dim <= 256 && p.memo_entries <= 8192 && p.rows > sms * many_per_sm(2) && p.rows <= sms * many_per_sm(1);
 }
 
 template <int LPR, int JP, int JU, int METRIC, bool ALIGNED>
 int pair_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)
 {
-    // a single warp needs 10 instead of 14 bytes of shared memory per candidate: rows of more than about 15,000 take it
-    if (vl_beam_solo(p) || many_layout<2, LPR, JP>(p).total > vl_smem_limit())
-        return many_launch<1, LPR, JP, JU, METRIC, ALIGNED>(p, row_order, launch, blocks, smem, stream);
+    // the choice described above; and a single warp needs 10 instead of 14 bytes of shared memory per candidate, so rows
+    // of more than about 15,000 candidates take it whatever their dimension
+    bool solo;
+    if (many_layout<2, LPR, JP>(p).total > vl_smem_limit()) solo = true;
+    else if (p.dim <= 128) solo = p.memo_entries <= 4096;
+    else solo = p.dim <= 256 && p.memo_entries <= 8192 && p.rows > rows_in_flight<2, LPR, JP, JU, METRIC, ALIGNED>(p) &&
+                p.rows <= rows_in_flight<1, LPR, JP, JU, METRIC, ALIGNED>(p);
+    if (solo) return many_launch<1, LPR, JP, JU, METRIC, ALIGNED>(p, row_order, launch, blocks, smem, stream);
     return many_launch<2, LPR, JP, JU, METRIC, ALIGNED>(p, row_order, launch, blocks, smem, stream);
 }
 
