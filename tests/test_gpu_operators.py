@@ -313,3 +313,24 @@ def test_prune_of_a_row_range_equals_the_full_prune_on_those_rows(built_lib):
     assert bool((out_b[:123] == -7).all()) and bool((out_b[377:] == -7).all())
     wb, wd = oracle.prune_(kn, d)
     assert np.array_equal(n(full_b), wb) and np.array_equal(n(full_d), wd)
+
+
+@pytest.mark.parametrize("dim", [64, 128, 768, 50])
+def test_distances_to_an_empty_set_are_sentinels(dim, built_lib):
+    """n = 0 with ids that are all MAXINT: sentinels, and nothing is read through `vectors`.  (That a row is not read cannot be
+    seen from its result, which is dropped: `vectors` is one allocated row of NaN here.)"""
+    import ctypes
+    from vectorlink_gpu import _lib
+    from vectorlink_gpu._lib import lib, ptr, stream_of
+    row = torch.full((dim,), float("nan"), device="cuda")
+    queries = torch.rand((3, dim), device="cuda")
+    none = torch.full((3, 5), 2147483647, dtype=torch.int32, device="cuda")
+    status = ptr(_lib.status_word("cuda"))
+    dist = torch.zeros((3, 5), device="cuda")
+    assert lib().vl_calculate_distances(ptr(row), 0, dim, ptr(queries), 3, ptr(none), 5, ptr(dist), 0, status, stream_of(row)) == 0
+    (ids, seeds) = (torch.zeros((3, 10), dtype=torch.int32, device="cuda"), torch.zeros((3, 10), device="cuda"))
+    assert lib().vl_search_from_seeds(ptr(queries), 3, ptr(none), 5, ptr(none), 2, ptr(row), 0, dim, ptr(ids), ptr(seeds), 0, status,
+                                      stream_of(row)) == 0
+    sentinel = torch.tensor(3.4028e37, device="cuda")
+    assert (dist == sentinel).all() and (seeds == sentinel).all() and (ids == 2147483647).all()
+    assert _lib.read_status("cuda") == 0

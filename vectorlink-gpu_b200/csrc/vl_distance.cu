@@ -145,7 +145,7 @@ template <int METRIC>
 int launch_gather(const GatherArgs& a, cudaStream_t stream)
 {
     const bool aligned = (a.dim % 4 == 0) && (((uintptr_t)a.vectors | (uintptr_t)a.queries) % 16 == 0);
-    if (aligned) {
+    if (aligned && a.n > 0) {      // the exact fit loads row 0 for a candidate that is none, so there has to be one
 #define VL_EXACT(L, J, U) if (a.dim == 4 * L * U) return gather_launch<L, J, U, METRIC, true>(a, stream);
         VL_EXACT(4, 4, 4)     // dim 64
         VL_EXACT(8, 4, 3)     // dim 96
