@@ -219,8 +219,12 @@ typedef struct vl_beam_params {
     unsigned long long* memo;  /* [memo_slots, memo_entries] scratch, any contents (see vl_beam_search_plan) */
     int64_t memo_slots;        /* rows in flight the scratch was sized for: >= blocks * rows_per_block of the plan */
     unsigned long long* stats; /* optional [16] counters (added to): [1] gathered candidates, [2] search-queue merges,
-                                  [3] visit-queue merges, [4] class-A candidates, [5] class-B rounds, [6] rows, [7] iterations */
-    int32_t flags;             /* ignored (a row's phases overlap, so they have no cycle counters of their own) */
+                                  [3] visit-queue merges, [4] class-A candidates, [5] class-B rounds, [6] rows, [7] iterations, [8..13] cycles
+                                  spent in: pop, neighbour ids + memo probe, gather + memo update, (0), choice of the entrants +
+                                  search-queue merge, visit-queue merge - by the clock of a row's first warp and, for the visit
+                                  queue, of its second one (the two merges of a row overlap) */
+    int32_t flags;             /* bit 0: also accumulate the per-phase cycle counters of `stats`; every row is then searched by
+                                  two warps and no batch ends together (launches of more than about 15,000 candidates per iteration have no such counters) */
     int32_t wait_us;           /* longest wait of one row for the others of its batch (vl_beam_search_rows with
                                   arrivals), in microseconds; <= 0 = 2 s */
     unsigned long long* row_ticket; /* optional device counter, zero at launch: warps then draw their next row from it

@@ -53,6 +53,27 @@ def test_one_or_two_warps_per_row_give_the_same_queues(count, memo, built_lib):
     assert torch.equal(fused[0], steps[0]) and torch.equal(fused[1], steps[1]) and fused[2] == steps[2]
 
 
+@pytest.mark.parametrize("count,dim", [(3, 64), (1300, 64), (1300, 512), (1300, 50)])
+def test_cycle_counters(count, dim, built_lib):
+    """The counters of every phase are there when they are asked for, in 16 words, and change nothing."""
+    import vectorlink_gpu.ann as A
+    ann = A.ANN(vectors=rows_of(1, 3001, dim, "cosine"), beam_size=16, visit_queue_factor=2, recall_search_queue_factor=2,
+                init="knn_tile", optimization_loops=1)
+    queries = rows_of(2, count, dim, "cosine")
+    want = ann.search(queries).indices.clone()
+    stats = {}
+    try:
+        for timers in (False, True):
+            (A.STATS, A.STATS_TIMERS) = (torch.zeros(24, dtype=torch.int64, device=DEV), timers)
+            assert torch.equal(ann.search(queries).indices, want)
+            stats[timers] = A.STATS.tolist()
+    finally:
+        (A.STATS, A.STATS_TIMERS) = (None, False)
+    assert stats[False][7] > 0 and stats[True][7] > 0
+    assert stats[False][8:] == [0] * 16
+    assert all(stats[True][i] > 0 for i in (8, 9, 10, 12, 13)) and stats[True][11] == 0 and stats[True][14:] == [0] * 10
+
+
 @pytest.mark.parametrize("width,memo_entries", [(16, 0), (48, 0), (52, 8192), (64, 0), (128, 0)])
 def test_one_warp_per_row_is_chosen_by_the_rows_that_fit(width, memo_entries, built_lib):
     """256 dimensions, where shared memory allows 20 or fewer rows per SM: the plan never leaves rows to a second wave because of

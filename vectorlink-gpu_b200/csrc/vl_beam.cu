@@ -55,6 +55,7 @@ int beam_dispatch(const vl_beam_params* pp, const int64_t* row_order, unsigned i
                  "vl_beam_search: memo_entries must be a power of two >= 2 and the memo 16-byte aligned");
     *blocks = *smem = 0;
     if (p.rows == 0) return 0;
+    if (vl_beam_timed_fits(p)) return vl_beam_timed_launch(p, row_order, launch, blocks, smem, stream);
     if (vl_beam_team_fits(p)) return launch ? vl_beam_team_launch(p, arrivals, stream) : 0;   // no scratch: *blocks stays 0
     return vl_beam_pair_launch(p, row_order, launch, blocks, smem, stream);
 }

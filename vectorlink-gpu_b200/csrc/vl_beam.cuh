@@ -53,6 +53,10 @@ __device__ __forceinline__ void memo_put(vl_key_t* memo, int buckets, int shift,
 // rows in flight, `smem`: bytes of shared memory of one.
 int vl_beam_pair_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream);
 
+// The same with two warps per row and cycle counters (vl_beam_timed.cu), if the launch asks for them and its rows fit.
+bool vl_beam_timed_fits(const vl_beam_params& p);
+int vl_beam_timed_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream);
+
 // A CTA of up to 16 warps per query row (vl_beam_team.cu), for launches of few rows; `arrivals` as in
 // vl_beam_search_rows.  The memo is on chip, no scratch is needed.
 bool vl_beam_team_fits(const vl_beam_params& p);

@@ -25,47 +25,9 @@
 // 2,368 searches 2.40 / 2.68, 2,500 3.47 / 2.79, 2,960 3.68 / 3.09, 3,100 3.81 / 5.05.  A second wave saved gains nothing (4,800,
 // 5,300, 5,900 searches 5.94 / 5.85, 6.05 / 6.21, 6.44 / 6.61; CTAs draw their next row as they finish, so waves blur); first round of
 // 20,000: 44.8 / 46.9; 768 dimensions lose (3,000 searches: 3.3 / 4.9).
-#include "vl_beam_team.cuh"
+#include "vl_beam_many.cuh"
 
 namespace {
-
-template <int TEAM, int LPR, int JP>
-TeamSmem many_layout(const vl_beam_params& p)
-{
-    return team_layout(p.pvc * p.graph_w, p.sq_len, p.vq_len, p.seen_cap, LPR * JP * 16, p.memo ? p.memo_entries : 0, false, TEAM > 1);
-}
-
-// CTAs = rows of this launch that the device keeps in flight at once; 0 if a row does not fit, -1 on an error
-template <int TEAM, int LPR, int JP, int JU, int METRIC, bool ALIGNED>
-int64_t rows_in_flight(const vl_beam_params& p)
-{
-    auto kernel = beam_team_kernel<LPR, JP, JU, METRIC, ALIGNED, TEAM>;
-    const TeamSmem lay = many_layout<TEAM, LPR, JP>(p);
-    if (lay.total > vl_smem_limit()) return 0;
-    int per_sm = 0;
-    if (vl_allow_smem(kernel) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 32 * TEAM, lay.total) != cudaSuccess) return -1;
-    return (int64_t)vl_sm_count() * per_sm;
-}
-
-template <int TEAM, int LPR, int JP, int JU, int METRIC, bool ALIGNED>
-int many_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)
-{
-    const TeamSmem lay = many_layout<TEAM, LPR, JP>(p);
-    VL_CHECK_ARG(lay.total <= vl_smem_limit(), "vl_beam_search: one row needs %d bytes of shared memory, the device offers %d", lay.total,
-                 vl_smem_limit());
-    const int64_t resident = rows_in_flight<TEAM, LPR, JP, JU, METRIC, ALIGNED>(p);   // one wave; further rows are drawn as CTAs finish
-    VL_CHECK_ARG(resident > 0, "vl_beam_search: occupancy query failed");
-    const int grid = (int)(p.rows < resident ? p.rows : resident);
-    *blocks = grid;
-    *smem = lay.total;
-    if (!launch) return 0;
-    VL_CHECK_ARG(!p.memo || p.memo_slots >= grid, "vl_beam_search: memo has %lld slots, the launch keeps %d rows in flight",
-                 (long long)p.memo_slots, grid);
-    beam_team_kernel<LPR, JP, JU, METRIC, ALIGNED, TEAM><<<grid, 32 * TEAM, lay.total, stream>>>(p, lay, row_order, nullptr);
-    VL_CHECK_LAUNCH("beam_team_kernel");
-    return 0;
-}
 
 template <int LPR, int JP, int JU, int METRIC, bool ALIGNED>
 int pair_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)

@@ -50,8 +50,11 @@ __host__ inline TeamSmem team_layout(int m, int sq_len, int vq_len, int seen_cap
 }
 
 // words of the control block: list lengths, real keys of the visit and the search queue, the end of the
-// batch, which buffer holds each queue, the next row
-enum { kTodo = 0, kListS, kListV, kQueued, kHeld, kStop, kSqBuf, kVqBuf, kRowLo, kRowHi, kWords };
+// batch, which buffer holds each queue, the cycle counters (the clock at the last phase of warp 0 and of the visit
+// queue's warp, then a sum per phase), and between two rows the next row
+enum { kTodo = 0, kListS, kListV, kQueued, kHeld, kStop, kSqBuf, kVqBuf, kClock, kClockV, kPop, kProbe, kGather, kSearchQ, kVisitQ, kWords,
+       kRowLo = kTodo, kRowHi = kListS };
+static_assert(kWords <= 16, "control block");
 
 __device__ __forceinline__ unsigned long long team_now_ns()
 {
@@ -232,7 +235,9 @@ __device__ __forceinline__ void team_gather(const vl_beam_params& p, uint2* cand
 // TEAM == kMaxTeam: launches of few rows, 2 to 16 warps per CTA (blockDim), the memo in shared memory.
 // JU > 0: exact-fit rows (dim == 4*LPR*JU, see vl_load_exact); JU == 0: any dimension, with 128-bit
 // loads when ALIGNED (dim % 4 == 0 and 16-byte aligned rows) and four scalar loads per chunk otherwise.
-template <int LPR, int JP, int JU, int METRIC, bool ALIGNED, int TEAM>
+// TIMED: with the cycle counters of `stats` (vl_beam_timed.cu).  A test of the launch's flags at every phase instead costs
+// launches without counters too: clusters of 30,000 x 96 9.16 / 9.44 ms, rounds 2 and 3 of 150,000 x 128 76, 78 / 82, 84.
+template <int LPR, int JP, int JU, int METRIC, bool ALIGNED, int TEAM, bool TIMED = false>
 __global__ void __launch_bounds__(TEAM * 32, TEAM <= 2 ? many_per_sm(TEAM) : 1)
 beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __restrict__ row_order, unsigned int* arrivals)
 {
@@ -257,6 +262,17 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
     const vl_key_t kSent = vl_sentinel_key();
     const uint32_t kPoppedOrd = 0xffffffffu;          // "popped" mark of a memo entry, above every real ordered distance
     const float inv_wb = 1.0f / (float)wb;
+    // TIMED: lane 0 of a warp adds the cycles since its last call to a phase (`sum`; kTodo = none, start only).
+    auto phase = [&](int since, int sum) {
+        if constexpr (TIMED) {
+            if (lane == 0) {
+                unsigned int now;
+                asm volatile("mov.u32 %0, %%clock;" : "=r"(now) : : "memory");
+                if (sum != kTodo) ctl[sum] = (int)((unsigned int)ctl[sum] + now - (unsigned int)ctl[since]);
+                ctl[since] = (int)now;
+            }
+        }
+    };
     // With a memo a candidate row is read about once per query row: unless rows are taken neighbourhood by
     // neighbourhood, stream it through L2 and keep the graph rows and the memo there instead.
     const uint64_t pol_stream = (TEAM <= 2 && p.memo && !row_order) ? vl_policy_evict_first() : vl_policy_evict_normal();
@@ -342,6 +358,7 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
 
 #pragma unroll 1
         for (; k <= n_run; ++k) {
+            if (warp == 0) phase(kClock, kTodo);
             const int first = (k - 1) * pvc;
             const bool seen_live = first < e_cap;    // utils.py:62-69
             const bool raw = p.dump_last && k == p.n_iters;   // needs every real distance
@@ -360,6 +377,7 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
             }
             const int ncopy = seen_live ? ((e_cap - first) < pvc ? (e_cap - first) : pvc) : 0;
             if (__any_sync(0xffffffffu, lane < ncopy && popped == VL_MAXINT)) always_full = false;
+            if (warp == 0) phase(kClock, kPop);
             // ---- neighbour ids (kernels.py:244), then which of them need a gather: live ids the memo does not know.
             // PB chunks per warp and round: the graph-row loads, then the memo loads, of a round are in flight together.
             constexpr int PB = TEAM <= 2 ? 6 : 4;
@@ -404,12 +422,14 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
                 }
             }
             __syncthreads();
+            if (warp == 0) phase(kClock, kProbe);
             // ---- gathered distances (kernels.py:248-257) ----
             const int n_todo = ctl[kTodo];
             st_todo += n_todo;
             team_gather<LPR, JP, JU, METRIC, ALIGNED, TEAM>(p, cand, todo, n_todo, q4, q, warp, nwarps, lane, pol_stream, memo,
                                                             lay.memo_buckets, lay.memo_shift, k & 1);
             __syncthreads();
+            if (warp == 0) phase(kClock, kGather);
             if (raw) { dumped = true; break; }
             // ---- which candidates can enter a queue: every warp looks at its share ----
             // Search queue: only candidates gathered now (a candidate the memo knew was offered when it was first
@@ -472,6 +492,7 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
                     }
                 }
                 __syncwarp();
+                phase(kClock, kSearchQ);
                 if (lane == 0) {
                     ctl[kTodo] = 0;
                     ctl[kListS] = 0;
@@ -509,6 +530,7 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
             }
             if (warp == (TEAM == 1 ? 0 : 1)) {
                 // ---- the popped heads leave, visit_queue.insert(..., exclude=seen) ----
+                phase(kClockV, kTodo);
                 if (TEAM == 1 && usual) {
 #pragma unroll 1
                     for (int c0 = 0; c0 < m_total; c0 += 32)
@@ -564,6 +586,7 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
                     ctl[kVqBuf] = vq == reinterpret_cast<vl_key_t*>(smem + lay.vq_a) ? lay.vq_a : lay.vq_b;
                 }
                 mark_popped(vq, k + 1);
+                phase(kClockV, kVisitQ);
             }
             __syncthreads();
             if (TEAM > 2 && ctl[kStop] != 0) {
@@ -605,6 +628,13 @@ beam_team_kernel(const vl_beam_params p, const TeamSmem lay, const int64_t* __re
                 atomicAdd(p.stats + 2, (unsigned long long)st_m);
                 atomicAdd(p.stats + 6, 1ull);
                 atomicAdd(p.stats + 7, (unsigned long long)(k <= n_run ? k : n_run));
+                if constexpr (TIMED) {
+                    atomicAdd(p.stats + 8, (unsigned long long)(unsigned int)ctl[kPop]);
+                    atomicAdd(p.stats + 9, (unsigned long long)(unsigned int)ctl[kProbe]);
+                    atomicAdd(p.stats + 10, (unsigned long long)(unsigned int)ctl[kGather]);
+                    atomicAdd(p.stats + 12, (unsigned long long)(unsigned int)ctl[kSearchQ]);
+                    atomicAdd(p.stats + 13, (unsigned long long)(unsigned int)ctl[kVisitQ]);
+                }
             }
             if (warp == (TEAM == 1 ? 0 : 1)) {
                 atomicAdd(p.stats + 3, (unsigned long long)st_v);

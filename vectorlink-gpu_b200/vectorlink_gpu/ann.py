@@ -30,9 +30,10 @@ FUSED_MAX_SMEM_PER_ROW = 200 * 1024
 # launching stream) and its count of distance evaluations: the benchmark's roofline figures.
 PROFILE = None
 PROFILE_TAG = "search"     # which phase the launches being profiled belong to (generate_ann sets it per round)
-# When set to an int64 CUDA tensor of 16 zeros, the fused kernel adds its work counters to it
-# (layout: `stats` in include/vlgpu.h).
+# When set to an int64 CUDA tensor of 16 zeros, the fused kernel adds its work counters and, with STATS_TIMERS,
+# per-phase cycles to it (layout: `stats` in include/vlgpu.h).
 STATS = None
+STATS_TIMERS = False
 
 
 def _metric_of(config: Dict):
@@ -119,7 +120,7 @@ def _launch_beam(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_len
     p.memo = 0
     p.memo_slots = 0
     p.stats = stats.data_ptr() if stats is not None else 0
-    p.flags = 0
+    p.flags = 1 if (stats is not None and stats is STATS and STATS_TIMERS) else 0
     p.wait_us = int(config.get("wait_us", 0))
     p.memo_entries = _memo_entries(p, config)
     smem, per_block, blocks = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
