@@ -10,12 +10,14 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.abspath(os.path.join(HERE, "..", "include"))
 OUT = os.path.join(HERE, "vectorlink_gpu", "libvlgpu.so")
-SOURCES = ["vl_api.cu", "vl_distance.cu", "vl_queue.cu", "vl_prune.cu", "vl_symmetrize.cu", "vl_components.cu", "vl_order.cu", "vl_beam.cu", "vl_beam_pair.cu", "vl_beam_timed.cu", "vl_beam_team.cu", "vl_knn_tile.cu"]
+SOURCES = ["vl_api.cu", "vl_distance.cu", "vl_queue.cu", "vl_prune.cu", "vl_symmetrize.cu", "vl_components.cu", "vl_order.cu", "vl_beam.cu", "vl_beam_pair.cu", "vl_beam_solo.cu", "vl_beam_timed.cu", "vl_beam_team.cu", "vl_knn_tile.cu"]
 
 
 def _stale() -> bool:
@@ -30,12 +32,16 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not _stale():
         return OUT
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    cmd = [nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-           "-I", INCLUDE, "-shared", "-Xcompiler", "-fPIC", "-o", OUT] + [os.path.join(CSRC, s) for s in SOURCES]
-    if verbose:
-        cmd.insert(1, "-Xptxas")
-        cmd.insert(2, "-v")
-    subprocess.check_call(cmd)
+    arch = [nvcc, "-gencode", "arch=compute_100a,code=sm_100a"]
+    options = ["-lineinfo", "-O3", "-std=c++17", "-I", INCLUDE, "-Xcompiler", "-fPIC"] + (["-Xptxas", "-v"] if verbose else [])
+    # one compiler per source, side by side: the beam search's files hold dozens of instantiations each
+    with tempfile.TemporaryDirectory() as objects, ThreadPoolExecutor(os.cpu_count() or 1) as pool:
+        def compile_one(source):
+            out = os.path.join(objects, source + ".o")
+            subprocess.check_call(arch + options + ["-c", "-o", out, os.path.join(CSRC, source)])
+            return out
+
+        subprocess.check_call(arch + ["-shared", "-Xcompiler", "-fPIC", "-o", OUT] + list(pool.map(compile_one, SOURCES)))
     return OUT
 
 

@@ -57,6 +57,7 @@ int beam_dispatch(const vl_beam_params* pp, const int64_t* row_order, unsigned i
     if (p.rows == 0) return 0;
     if (vl_beam_timed_fits(p)) return vl_beam_timed_launch(p, row_order, launch, blocks, smem, stream);
     if (vl_beam_team_fits(p)) return launch ? vl_beam_team_launch(p, arrivals, stream) : 0;   // no scratch: *blocks stays 0
+    if (vl_beam_one_warp(p)) return vl_beam_solo_launch(p, row_order, launch, blocks, smem, stream);
     return vl_beam_pair_launch(p, row_order, launch, blocks, smem, stream);
 }
 

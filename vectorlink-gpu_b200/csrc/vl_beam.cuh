@@ -49,9 +49,12 @@ __device__ __forceinline__ void memo_put(vl_key_t* memo, int buckets, int shift,
 
 }  // namespace
 
-// Two warps per query row (vl_beam_pair.cu).  Plans the launch and, with `launch`, runs it; `blocks`: CTAs =
-// rows in flight, `smem`: bytes of shared memory of one.
+// Two warps per query row (vl_beam_pair.cu) or one (vl_beam_solo.cu).  Each plans the launch and, with `launch`, runs it;
+// `blocks`: CTAs = rows in flight, `smem`: bytes of shared memory of one.
+bool vl_beam_one_warp(const vl_beam_params& p);          // which of the two a launch takes
+int64_t vl_beam_solo_rows(const vl_beam_params& p);      // rows that one warp each keeps in flight
 int vl_beam_pair_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream);
+int vl_beam_solo_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream);
 
 // The same with two warps per row and cycle counters (vl_beam_timed.cu), if the launch asks for them and its rows fit.
 bool vl_beam_timed_fits(const vl_beam_params& p);

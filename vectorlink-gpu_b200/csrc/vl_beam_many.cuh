@@ -1,5 +1,5 @@
 // Launches of the fused beam search that keep as many rows in flight as fit, memos in global memory, one or two
-// warps per row: shared by vl_beam_pair.cu and vl_beam_timed.cu.
+// warps per row: shared by vl_beam_pair.cu, vl_beam_solo.cu and vl_beam_timed.cu.
 #pragma once
 #include "vl_beam_team.cuh"
 

@@ -1,5 +1,5 @@
-// Fused beam search with two warps per query row and 16 rows in flight per SM, or one warp and 20 rows:
-// launches of many rows.
+// Fused beam search with two warps per query row and 16 rows in flight per SM, or one warp (vl_beam_solo.cu) and 20
+// rows: launches of many rows.
 //
 // A row's iteration is a chain of memory round trips and queue steps, so a launch is bound by latency
 // at the number of rows that can be in flight.  That number is bound in turn by the rows' memos
@@ -30,20 +30,36 @@
 namespace {
 
 template <int LPR, int JP, int JU, int METRIC, bool ALIGNED>
+bool pair_fits(const vl_beam_params& p)
+{
+    return many_layout<2, LPR, JP>(p).total <= vl_smem_limit();
+}
+
+template <int LPR, int JP, int JU, int METRIC, bool ALIGNED>
+int64_t pair_rows(const vl_beam_params& p)
+{
+    return rows_in_flight<2, LPR, JP, JU, METRIC, ALIGNED>(p);
+}
+
+template <int LPR, int JP, int JU, int METRIC, bool ALIGNED>
 int pair_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)
 {
-    // the choice described above; and a single warp needs 10 instead of 14 bytes of shared memory per candidate, so rows
-    // of more than about 15,000 candidates take it whatever their dimension
-    bool solo;
-    if (many_layout<2, LPR, JP>(p).total > vl_smem_limit()) solo = true;
-    else if (p.dim <= 128) solo = p.memo_entries <= 4096;
-    else solo = p.dim <= 256 && p.memo_entries <= 8192 && p.rows > rows_in_flight<2, LPR, JP, JU, METRIC, ALIGNED>(p) &&
-                p.rows <= rows_in_flight<1, LPR, JP, JU, METRIC, ALIGNED>(p);
-    if (solo) return many_launch<1, LPR, JP, JU, METRIC, ALIGNED>(p, row_order, launch, blocks, smem, stream);
     return many_launch<2, LPR, JP, JU, METRIC, ALIGNED>(p, row_order, launch, blocks, smem, stream);
 }
 
+bool two_warps_fit(const vl_beam_params& p) { VL_BEAM_DISPATCH(p, pair_fits, p); }
+int64_t two_warp_rows(const vl_beam_params& p) { VL_BEAM_DISPATCH(p, pair_rows, p); }
+
 }  // namespace
+
+// the choice described above; and a single warp needs 10 instead of 14 bytes of shared memory per candidate, so rows
+// of more than about 15,000 candidates take it whatever their dimension
+bool vl_beam_one_warp(const vl_beam_params& p)
+{
+    if (!two_warps_fit(p)) return true;
+    if (p.dim <= 128) return p.memo_entries <= 4096;
+    return p.dim <= 256 && p.memo_entries <= 8192 && p.rows > two_warp_rows(p) && p.rows <= vl_beam_solo_rows(p);
+}
 
 int vl_beam_pair_launch(const vl_beam_params& p, const int64_t* row_order, bool launch, int* blocks, int* smem, cudaStream_t stream)
 {
