@@ -137,3 +137,24 @@ def test_a_plan_of_another_thread_does_not_refuse_a_launch(built_lib):
         stop.set()
         planner.join()
     assert not refused and blocks.value > 0
+
+
+def test_the_seed_table_outlives_its_place_in_the_cache(built_lib):
+    """A table that leaves the cache while another stream has yet to read it: its memory is not given to anyone before."""
+    from vectorlink_gpu import utils
+    utils._sorted_primes.cache_clear()
+    want = utils.seed_offsets(700, DEV).clone()
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(400_000_000)
+        table = utils.seed_offsets(700, DEV)
+        at = table.data_ptr()
+        read = table + 0
+    del table
+    utils._sorted_primes.cache_clear()
+    others = [torch.full((700,), -1, dtype=torch.int32, device=DEV) for _ in range(3000)]
+    early = not side.query()                 # all of them were made while the other stream had still to read
+    torch.cuda.synchronize()
+    assert torch.equal(read, want)
+    assert not early or all(o.data_ptr() != at for o in others)

@@ -42,7 +42,10 @@ def _sorted_primes(size: int, device: torch.device) -> Tensor:
 
 def seed_offsets(size: int, device) -> Tensor:
     """The first `size` seed offsets in rising order: a constant table, kept per size and device."""
-    return _sorted_primes(size, _lib._device_key(device))
+    table = _sorted_primes(size, _lib._device_key(device))
+    # it may leave the cache while kernels of this stream still have to read it
+    table.record_stream(torch.cuda.current_stream(table.device))
+    return table
 
 
 def generate_queue_circulants(batch_size: int, num_vecs: int, primes: Tensor, first_row: int = 0) -> Tensor:
