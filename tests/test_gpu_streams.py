@@ -158,3 +158,21 @@ def test_the_seed_table_outlives_its_place_in_the_cache(built_lib):
     torch.cuda.synchronize()
     assert torch.equal(read, want)
     assert not early or all(o.data_ptr() != at for o in others)
+
+
+def test_the_status_word_is_zero_before_another_stream_sets_a_bit(built_lib):
+    from vectorlink_gpu import _lib
+    from vectorlink_gpu.kernels import calculate_distances
+    vectors = unit_rows(1, 10, 64)
+    bad = torch.full((10, 1), 99, dtype=torch.int32, device=DEV)      # no such row: skipped and reported
+    calculate_distances(vectors, bad)
+    assert _lib.read_status(DEV) == 1
+    torch.cuda.synchronize()
+    _lib._status.clear()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        torch.cuda._sleep(200_000_000)
+        _lib.status_word(DEV)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        calculate_distances(vectors, bad)
+    torch.cuda.synchronize()
+    assert _lib.read_status(DEV) == 1

@@ -134,7 +134,9 @@ def status_word(device) -> torch.Tensor:
     """One int32 per device that kernels OR VL_STATUS_* bits into."""
     key = _device_key(device)
     if key not in _status:
-        _status[key] = torch.zeros(1, dtype=torch.int32, device=key)
+        word = torch.zeros(1, dtype=torch.int32, device=key)
+        torch.cuda.current_stream(key).synchronize()     # zero before a kernel of another stream sets a bit
+        _status.setdefault(key, word)                    # of two threads that make it, one has its word used
     return _status[key]
 
 
