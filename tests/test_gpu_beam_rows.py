@@ -255,6 +255,28 @@ def test_row_order_of_a_build_changes_nothing(built_lib):
     assert torch.equal(graphs[0][0], graphs[1][0]) and torch.equal(graphs[0][1], graphs[1][1])
 
 
+def test_profiled_launches_include_their_row_order(built_lib):
+    import vectorlink_gpu.ann as A
+    vectors = rows_of(7, 3000, 48, "cosine")
+    config = dict(A.ANN(vectors=vectors[:64].contiguous(), beam_size=8).configuration, memo=True, optimization_loops=1)
+    real = A._row_order
+
+    def slow_order(graph, self_base, rows, config):
+        if self_base >= 0:
+            torch.cuda._sleep(100_000_000)              # 50 ms at 2 GHz
+        return real(graph, self_base, rows, config)
+
+    A._row_order = slow_order
+    A.PROFILE = []
+    try:
+        A.generate_ann(vectors, config)
+        torch.cuda.synchronize()
+        ms = [p["start"].elapsed_time(p["end"]) for p in A.PROFILE if p["tag"] == "round0"]
+    finally:
+        (A._row_order, A.PROFILE) = (real, None)
+    assert ms and ms[0] > 40
+
+
 @pytest.mark.parametrize("n,w,lo,hi", [(1, 1, 0, 1), (50, 7, 10, 50), (3000, 96, 0, 3000)])
 def test_locality_keys(n, w, lo, hi, built_lib):
     from vectorlink_gpu._lib import lib, ptr, stream_of

@@ -27,7 +27,8 @@ from .utils import add_new_to_seen_, generate_circulant_beams, generate_queue_ci
 
 FUSED_MAX_SMEM_PER_ROW = 200 * 1024
 # When set to a list, every fused-kernel launch appends its CUDA events (recorded on the
-# launching stream) and its count of distance evaluations: the benchmark's roofline figures.
+# launching stream; the making of the row order is between them) and its count of distance evaluations: the
+# benchmark's roofline figures.
 PROFILE = None
 PROFILE_TAG = "search"     # which phase the launches being profiled belong to (generate_ann sets it per round)
 # When set to an int64 CUDA tensor of 16 zeros, the fused kernel adds its work counters and, with STATS_TIMERS,
@@ -137,11 +138,11 @@ def _launch_beam(vectors, graph, queries, seed_ids, seed_dist, seed_cols, sq_len
         memo = torch.empty(slots * p.memo_entries, dtype=torch.int64, device=vectors.device)
         p.memo = memo.data_ptr()
         p.memo_slots = slots
-    order = _row_order(graph, self_base, queries.size(0), config) if p.memo else None
-    if PROFILE is not None:
+    if PROFILE is not None:         # the row order is part of what the launch costs
         start = torch.cuda.Event(enable_timing=True)
         end = torch.cuda.Event(enable_timing=True)
         start.record()
+    order = _row_order(graph, self_base, queries.size(0), config) if p.memo else None
     check(lib().vl_beam_search_rows(ctypes.byref(p), ptr(order), ptr(arrivals), stream_of(vectors)), "vl_beam_search_rows")
     if PROFILE is not None:
         end.record()
