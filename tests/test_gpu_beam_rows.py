@@ -277,6 +277,14 @@ def test_profiled_launches_include_their_row_order(built_lib):
     assert ms and ms[0] > 40
 
 
+def test_first_row_as_a_float(built_lib):
+    """Row numbers were and are taken as torch.arange takes them."""
+    from vectorlink_gpu import ANN
+    ann = ANN(vectors=rows_of(1, 500, 32, "cosine"), beam_size=8, optimization_loops=1)
+    queries = rows_of(2, 3, 32, "cosine")
+    assert torch.equal(ann.search(queries, first_row=7.0).indices, ann.search(queries, first_row=7).indices)
+
+
 @pytest.mark.parametrize("n,w,lo,hi", [(1, 1, 0, 1), (50, 7, 10, 50), (3000, 96, 0, 3000)])
 def test_locality_keys(n, w, lo, hi, built_lib):
     from vectorlink_gpu._lib import lib, ptr, stream_of

@@ -68,7 +68,7 @@ def circulant_seeds(vectors: Tensor, queries: Tensor, offsets: Tensor, first_row
     ids = torch.empty((rows, w), dtype=torch.int32, device=vectors.device)
     dist = torch.empty((rows, w), dtype=torch.float32, device=vectors.device)
     check(lib().vl_circulant_seeds(ptr(vectors), ctypes.c_int64(vectors.size(0)), vectors.size(1), ptr(queries),
-                                   ctypes.c_int64(rows), ptr(offsets), w, ctypes.c_int64(first_row), ctypes.c_int64(modulo),
+                                   ctypes.c_int64(rows), ptr(offsets), w, ctypes.c_int64(int(first_row)), ctypes.c_int64(modulo),
                                    ptr(ids), ptr(dist), metric_code(metric), ptr(_lib.status_word(vectors.device)),
                                    stream_of(vectors)), "vl_circulant_seeds")
     return ids, dist
