@@ -196,6 +196,39 @@ def launches_of(ann, queries):
         A.PROFILE = None
 
 
+# 8 warps per row and one row per SM, 8 and two, 4 and four, 2 and eight; 16 warps where an iteration has 256 candidates
+@pytest.mark.parametrize("count,degree", [(100, 16), (200, 16), (500, 16), (1000, 16), (100, 64)])
+@pytest.mark.parametrize("exclude_w", [0, 2])
+def test_larger_batches_that_stop_early_end_together(count, degree, exclude_w, built_lib):
+    import vectorlink_gpu.ann as A
+    ann = converging_index(degree, 64)
+    queries = flat_rows(4, count, 64)
+    exclude = ann.search(queries).indices[:, :exclude_w].contiguous() if exclude_w else None
+    got = []
+    for more in ({}, {"stepwise": True}):
+        queue = A.initial_search_queue(ann.vectors, queries, ann.configuration)
+        A.PROFILE = []
+        try:
+            A.closest_vectors(queries, queue, ann.vectors, ann.beams, dict(ann.configuration, **more), exclude)
+            launches = len(A.PROFILE)
+        finally:
+            A.PROFILE = None
+        assert launches == (0 if more else 1)
+        got.append((queue.indices, queue.distances, A.closest_vectors.last_count))
+    assert got[1][2] <= A.loop_bounds(ann.configuration)[0]
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]) and got[0][2] == got[1][2]
+
+
+# dimensions whose oracle cases are too few rows for the launches of many
+@pytest.mark.parametrize("metric,dim", [("cosine", 384), ("l2", 384), ("cosine", 512), ("l2", 512), ("cosine", 1536), ("l2", 2052), ("cosine", 1024)])
+def test_many_rows_of_wide_vectors(metric, dim, built_lib):
+    from vectorlink_gpu import ANN
+    ann = ANN(vectors=rows_of(1, 2001, dim, metric), beam_size=16, visit_queue_factor=2, recall_search_queue_factor=2,
+              metric=metric, init="knn_tile", optimization_loops=1)
+    (fused, steps) = search_both_ways(ann, rows_of(2, 1300, dim, metric))
+    assert torch.equal(fused[0], steps[0]) and torch.equal(fused[1], steps[1]) and fused[2] == steps[2]
+
+
 @pytest.mark.parametrize("count", [200, 500, 1000])
 def test_a_wait_that_runs_out_is_answered_by_a_second_run(count, built_lib):
     """Rows of a batch wait at most a microsecond for the others: some give up, and the batch is searched again without
