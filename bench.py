@@ -249,10 +249,11 @@ def launch_classes(profile, reps, dim):
 
 
 def dram_captures(workload):
-    """ncu DRAM counters of earlier captures of this workload, kept as data beside the summaries."""
+    """ncu DRAM counters of earlier captures of this workload, kept as data beside the summaries; only those of the kernel
+    that runs now (none is on record at present)."""
     try:
         doc = json.load(open(os.path.join(ROOT, "profiles", "dram_traffic.json")))
-        return [c for c in doc["captures"] if c["workload"] == workload]
+        return [c for c in doc["captures"] if c["workload"] == workload and c["kernel"].startswith("beam_team_kernel")]
     except Exception:
         return []
 
@@ -265,8 +266,9 @@ def roofline_of(build_classes, search_classes, peak, peak_kind, workload, dim, k
         bandwidth of the gather, whichever level of the memory system served it;
     `dram` - DRAM bytes of an ncu capture of the same launch class (scaled by gathered rows).
     The headline `achieved`/`frac` is `gathered` of the build's later rounds, whose rows come from
-    DRAM; the first round's candidates lie in a band of rows that stays in L2, so its `gathered`
-    figure is an L2 rate and is reported but not used as the HBM fraction."""
+    DRAM or, where rows in flight together share them, from L2: a gather rate, which only a capture turns into
+    a share of the HBM bandwidth.  The first round's candidates lie in a band of rows that stays in L2, so its
+    `gathered` figure is an L2 rate and is reported but not used as the headline."""
     classes = {}
     caps = dram_captures(workload)
     for cls, c in list(build_classes.items()) + [("search", search_classes.get("search"))]:
