@@ -196,7 +196,7 @@ typedef struct vl_beam_params {
     const float* seed_dist;    /*   empty queue (= Queue.insert of ann.py:147 / the head of a Queue) */
     int64_t seed_ld;
     int32_t seed_cols;
-    int32_t sq_len;            /* search queue length, <= 1024 */
+    int32_t sq_len;            /* search queue length, <= 4096 */
     int32_t vq_len;            /* visit queue length = visit_queue_factor * beam_size, >= pvc */
     int32_t seen_cap;          /* exclude_factor * vq_len */
     int32_t* out_ids;          /* [rows, out_ld]: out_cols columns written per row: the head, then */

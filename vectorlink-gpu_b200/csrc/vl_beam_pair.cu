@@ -8,7 +8,7 @@
 // by side at 64 registers per thread, without another row's memo.  Build rounds, ms, one warp per row with
 // the queue merges of before (128 registers) / this, rows in neighbourhood order, on one B200:
 //   1,000,000 x 128, lists of 96 from near neighbours: 660 / 526
-//   60,007 x 768, lists of 192:                        155 / 121
+//   60,007 x 768, lists of 192:                        155 / 121  (shared memory holds 9 of these rows per SM, also below)
 //   150,000 x 128, rounds 2 and 3:                  98, 97 / 76, 78
 // 10,000 searches of 1,000,000 x 128: 6.6 / 5.3; 2,500 of 200,000 x 256: 2.33 / 1.55.  12 rows per SM at 80
 // registers (two gather steps in flight): 541, 119, 81; one warp per row with the same queue step at 16 rows per
