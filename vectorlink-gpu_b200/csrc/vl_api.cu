@@ -31,11 +31,15 @@ int vl_sm_count()
     return cached[dev];
 }
 
+// asked once per device, like the SMs
 int vl_smem_limit()
 {
+    static int cached[64] = {0};
     int dev = 0, bytes = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev < 64 && cached[dev] != 0) return cached[dev];
+    if (cudaDeviceGetAttribute(&bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
+    if (dev < 64) cached[dev] = bytes;
     return bytes;
 }
 
